@@ -101,6 +101,10 @@ ZB_DEVICE void prefetch_tmap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// 2-D FP64 tensor map over a column-major matrix (host side, gemm_f64_tma.cu): box 16 x box_outer
+// elements with 128-byte swizzle; out-of-range elements read 0.
+cudaError_t make_f64_map(CUtensorMap* map, const double* base, long inner, long outer, long ld, int box_outer);
+
 // ----------------------------------------------------------------- tcgen05
 ZB_DEVICE void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(dst_smem)),
@@ -190,6 +194,27 @@ cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t s
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+
+// launch_dependent with a cluster shape given at launch.
+template <typename... P, typename... A>
+cudaError_t launch_dependent_cluster(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                     dim3 cluster, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster.x;
+    attr[1].val.clusterDim.y = cluster.y;
+    attr[1].val.clusterDim.z = cluster.z;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 

@@ -266,22 +266,6 @@ dgemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
 }
 
-// 2-D FP64 tensor map over a column-major matrix with `inner` contiguous
-// elements per column (leading dimension ld) and `outer` columns; box
-// 16 x box_outer elements with 128-byte swizzle; out-of-range elements read 0.
-cudaError_t make_f64_map(CUtensorMap* map, const double* base, long inner, long outer, long ld, int box_outer) {
-    auto enc = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(tensor_map_encoder());
-    if (!enc) return cudaErrorNotSupported;
-    cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
-    cuuint64_t strides[1] = {(cuuint64_t)(ld * 8)};
-    cuuint32_t box[2] = {16, (cuuint32_t)box_outer};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(base), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-
 template <bool A_MN, bool B_K, bool PARTIAL>
 cudaError_t launch_tma(const CUtensorMap& ma, const CUtensorMap& mb, const TmaGemmParams& P, int splits,
                        cudaStream_t st) {
@@ -306,6 +290,22 @@ cudaError_t dispatch_tma(bool a_mn, bool b_k, const CUtensorMap& ma, const CUten
 }
 
 }  // namespace
+
+// 2-D FP64 tensor map over a column-major matrix with `inner` contiguous
+// elements per column (leading dimension ld) and `outer` columns; box
+// 16 x box_outer elements with 128-byte swizzle; out-of-range elements read 0.
+cudaError_t make_f64_map(CUtensorMap* map, const double* base, long inner, long outer, long ld, int box_outer) {
+    auto enc = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(tensor_map_encoder());
+    if (!enc) return cudaErrorNotSupported;
+    cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
+    cuuint64_t strides[1] = {(cuuint64_t)(ld * 8)};
+    cuuint32_t box[2] = {16, (cuuint32_t)box_outer};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(base), dims, strides, box, estr,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
 
 bool dgemm_tma_applies(const GemmArgsF64& g) {
     const uintptr_t bits = reinterpret_cast<uintptr_t>(g.a) | reinterpret_cast<uintptr_t>(g.b);

@@ -49,6 +49,7 @@ enum TileShape : int {
 struct GemmPlan {
     int tile = TILE_128x128;
     int splits = 1;  // > 1: split-K over `splits` K ranges, needs a workspace
+    bool automatic = true;  // false: `splits` was asked for by the caller and is kept
 };
 
 // Workspace (in elements of T) a plan needs.
@@ -66,6 +67,10 @@ cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* wor
 bool dgemm_tma_applies(const GemmArgsF64& g);
 int dgemm_tma_k_chunk(int k, int splits);
 cudaError_t dgemm_tma(const GemmArgsF64& g, int splits, double* workspace, cudaStream_t st);
+// Warp-specialised 64 x 64 DGEMM tiles (gemm_f64_ws.cu), K split over the CTAs of a
+// cluster of `splits` (1 or 2) that sum their partial tiles through distributed
+// shared memory: no workspace.  Needs dgemm_tma_applies(g).
+cudaError_t dgemm_ws(const GemmArgsF64& g, int splits, cudaStream_t st);
 // K ranges dgemm_native will actually use for this plan (1: no workspace); the
 // route (GEMV, tall-skinny, tiles) and the rounding of K slices can only lower
 // it below plan.splits.

@@ -96,7 +96,10 @@ extern "C" int zynum_blas_gpu_dgemm_noalloc_device(char transa, char transb, int
         return -(int)e;
     }
     GemmPlan plan = plan_native_gemm(m, n, k, 8, sms);
-    if (splits > 0) plan.splits = splits < kMaxForcedSplits ? splits : kMaxForcedSplits;
+    if (splits > 0) {
+        plan.splits = splits < kMaxForcedSplits ? splits : kMaxForcedSplits;
+        plan.automatic = false;
+    }
     GemmArgsF64 g{ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc};
     // scratch only for the partial sums of the K ranges the route really uses
     // (the tall-skinny route uses none; K slices are rounded up, which can
