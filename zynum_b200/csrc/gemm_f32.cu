@@ -9,7 +9,13 @@
 // IEEE FP32 has no exact tensor-core kind (kind::tf32 drops mantissa bits), so
 // the native SGEMM is a CUDA-core FFMA kernel: 128 x 128 block tile, 256
 // threads, an 8 x 8 register tile per thread split into two 4-row and two
-// 4-column halves so that every shared load is a conflict-free float4.
+// 4-column halves so that every shared load is a conflict-free float4.  Two
+// rows of a column share one fma.rn.f32x2 (each half rounded as fmaf, so the
+// result is the same bit for bit): scalar FFMA was issue-bound at 85 % of the
+// slots, packed it takes half of them and the register file's operand reads
+// bound it (a register-only loop of this tile reaches 59.5 TFLOP/s packed, with
+// op(B)'s element duplicated by moves as here, and 49 scalar).  4096^3: 2654 ->
+// 2543 us (54.0 TFLOP/s), 8192^3 NT 53.7 -> 56.1 TFLOP/s.
 // Operands are staged with cp.async; a K-fast global operand (op = T for A,
 // op = N for B) is transposed on the fly by per-element copies.
 #include <algorithm>
@@ -99,6 +105,19 @@ struct TileLoader {
     }
 };
 
+// Two independent FP32 fused multiply-adds in one instruction, each rounded as fmaf.
+ZB_DEVICE void fma_f32x2(uint64_t& d, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(a), "l"(b));
+}
+ZB_DEVICE uint64_t pack_f32x2(float x, float y) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+ZB_DEVICE void unpack_f32x2(uint64_t v, float& x, float& y) {
+    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(x), "=f"(y) : "l"(v));
+}
+
 // Thread (tx, ty) owns rows {ty*4 + i, 64 + ty*4 + i} and columns
 // {64 q + tx*4 + j}, q < BN / 64; a warp covers 4 ty x 8 tx, so each float4
 // fragment load touches 4 (A) or 8 (B) distinct 16-byte words: one
@@ -126,11 +145,12 @@ sgemm_ffma_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __
 
     const uint32_t a_valid = LA::init(m0, M), b_valid = LB::init(n0, N);
 
-    float acc[8][JN];
+    // acc2[p][j]: rows (2p, 2p + 1) of the thread's eight and column j, as one packed pair
+    uint64_t acc2[4][JN];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int p = 0; p < 4; ++p)
 #pragma unroll
-        for (int j = 0; j < JN; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < JN; ++j) acc2[p][j] = 0ull;
 
     auto load_stage = [&](int stage, int kt) {
         const int k0 = kb + kt * BK;
@@ -162,19 +182,27 @@ sgemm_ffma_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __
         const float* bs = Bs + (kt % STAGES) * BK * PB;
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
-            float a[8], b[JN];
-            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(as + kk * PA + ty * 4);
-            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(as + kk * PA + 64 + ty * 4);
+            uint64_t a2[4];
+            float b[JN];
+            *reinterpret_cast<ulonglong2*>(a2) = *reinterpret_cast<const ulonglong2*>(as + kk * PA + ty * 4);
+            *reinterpret_cast<ulonglong2*>(a2 + 2) = *reinterpret_cast<const ulonglong2*>(as + kk * PA + 64 + ty * 4);
 #pragma unroll
             for (int q = 0; q < JN / 4; ++q)
                 *reinterpret_cast<float4*>(b + 4 * q) = *reinterpret_cast<const float4*>(bs + kk * PB + 64 * q + tx * 4);
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+            for (int j = 0; j < JN; ++j) {
+                const uint64_t bb = pack_f32x2(b[j], b[j]);
 #pragma unroll
-                for (int j = 0; j < JN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int p = 0; p < 4; ++p) fma_f32x2(acc2[p][j], a2[p], bb);
+            }
         }
     }
     cp_async_wait<0>();
+    float acc[8][JN];
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int j = 0; j < JN; ++j) unpack_f32x2(acc2[p][j], acc[2 * p][j], acc[2 * p + 1][j]);
 
     // Rows ty*4 .. ty*4+3 of one column are contiguous in column-major C:
     // one 16-byte access when the destination allows it.
