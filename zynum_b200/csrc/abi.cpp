@@ -157,8 +157,9 @@ cudaError_t run_gemm(const GemmArgsF64& g, cudaStream_t st, HostScratch s) { ret
 cudaError_t run_gemm(const GemmArgsF32& g, cudaStream_t st, HostScratch s) { return run_sgemm(g, st, s); }
 
 // Large host GEMMs run as column panels of C over three streams: the upload
-// stream copies A and then, panel by panel, B (and C when beta != 0); the
-// compute stream runs a panel's GEMM once its inputs are in; each C panel is
+// stream copies A and then, panel by panel, B (and C when beta != 0; pageable
+// matrices through the pinned slots of CopyTeam); the compute stream runs a
+// panel's GEMM once its inputs are in; each C panel is
 // downloaded on the download stream as soon as the host has seen its GEMM
 // finish without error.  Uploads, products and downloads of different panels
 // overlap (the link is full duplex).  Every device buffer is reserved before
@@ -206,24 +207,8 @@ void host_gemm_panels(const char* routine, Context& cx, int panels, char ta, cha
     };
     for (auto& x : ev)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
-    // uploads: A, then per panel op(B)[:, j0:j1] (and C[:, j0:j1]); in_j after panel j
-    if (e == cudaSuccess)
-        e = cudaMemcpy2DAsync(da, (size_t)ra * es, a, (size_t)lda * es, (size_t)ra * es, ca, cudaMemcpyHostToDevice,
-                              up);
-    for (int j = 0; j < panels && e == cudaSuccess; ++j) {
-        const int j0 = j * nb, w = std::min(nb, n - j0);
-        if (tb == 'N')  // B is k x n: columns j0 .. j0 + w
-            e = cudaMemcpy2DAsync(db + (long)j0 * rb, (size_t)rb * es, b + (long)j0 * ldb, (size_t)ldb * es,
-                                  (size_t)rb * es, w, cudaMemcpyHostToDevice, up);
-        else  // B is n x k: rows j0 .. j0 + w
-            e = cudaMemcpy2DAsync(db + j0, (size_t)rb * es, b + j0, (size_t)ldb * es, (size_t)w * es, k,
-                                  cudaMemcpyHostToDevice, up);
-        if (e == cudaSuccess && beta != T(0))
-            e = cudaMemcpy2DAsync(dc + (long)j0 * m, (size_t)m * es, c + (long)j0 * ldc, (size_t)ldc * es,
-                                  (size_t)m * es, w, cudaMemcpyHostToDevice, up);
-        if (e == cudaSuccess) e = cudaEventRecord(ev[2 * j], up);
-    }
-    // products.  FP64 through the CRT Ozaki scheme: one plan for the full panel width,
+    CopyTeam team(cx.slots, cx.device);
+    // FP64 through the CRT Ozaki scheme: one plan for the full panel width,
     // op(A)'s residues computed by the first panel and reused by the others (its row
     // scaling depends on op(A) alone, each column of op(B) is scaled independently, so
     // the result equals the unpanelled product's)
@@ -240,9 +225,21 @@ void host_gemm_panels(const char* routine, Context& cx, int panels, char ta, cha
     }
     void* ows = nullptr;
     if (crt && e == cudaSuccess) e = HostScratch{&cx}(ozaki_workspace_bytes(op), st, &ows);
+    // uploads: A, then per panel op(B)[:, j0:j1] (and C[:, j0:j1]), ev[2 j] after panel j; each
+    // panel's product is enqueued as soon as its uploads are
+    if (e == cudaSuccess) e = team.upload(da, (size_t)ra * es, a, (size_t)lda * es, (size_t)ra * es, ca, up);
     for (int j = 0; j < panels && e == cudaSuccess; ++j) {
         const int j0 = j * nb, w = std::min(nb, n - j0);
-        e = cudaStreamWaitEvent(st, ev[2 * j], 0);
+        if (tb == 'N')  // B is k x n: columns j0 .. j0 + w
+            e = team.upload(db + (long)j0 * rb, (size_t)rb * es, b + (long)j0 * ldb, (size_t)ldb * es, (size_t)rb * es, w,
+                            up);
+        else  // B is n x k: rows j0 .. j0 + w
+            e = team.upload(db + j0, (size_t)rb * es, b + j0, (size_t)ldb * es, (size_t)w * es, k, up);
+        if (e == cudaSuccess && beta != T(0))
+            e = team.upload(dc + (long)j0 * m, (size_t)m * es, c + (long)j0 * ldc, (size_t)ldc * es, (size_t)m * es, w,
+                            up);
+        if (e == cudaSuccess) e = cudaEventRecord(ev[2 * j], up);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ev[2 * j], 0);
         if (e != cudaSuccess) break;
         const T* bj = (tb == 'N') ? db + (long)j0 * rb : db + j0;
         GemmArgs<T> g{ta, tb, m, w, k, alpha, da, ra, bj, rb, beta, dc + (long)j0 * m, m};
@@ -268,8 +265,8 @@ void host_gemm_panels(const char* routine, Context& cx, int panels, char ta, cha
             report_gpu_failure(routine);
             return;
         }
-        e = cudaMemcpy2DAsync(c + (long)j0 * ldc, (size_t)ldc * es, dc + (long)j0 * m, (size_t)m * es,
-                              (size_t)m * es, w, cudaMemcpyDeviceToHost, down);
+        e = team.download(c + (long)j0 * ldc, (size_t)ldc * es, dc + (long)j0 * m, (size_t)m * es, (size_t)m * es, w,
+                          down);
         if (e != cudaSuccess) break;
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(down);
@@ -320,14 +317,13 @@ void host_gemm(const char* routine, char ta, char tb, int m, int n, int k, T alp
         host_gemm_panels<T>(routine, cx, panels, ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, da, db, dc);
         return;
     }
+    CopyTeam team(cx.slots, cx.device);
     if (!quick) {
-        e = cudaMemcpy2DAsync(da, (size_t)ra * es, a, (size_t)lda * es, (size_t)ra * es, ca, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess)
-            e = cudaMemcpy2DAsync(db, (size_t)rb * es, b, (size_t)ldb * es, (size_t)rb * es, cb, cudaMemcpyHostToDevice,
-                                  st);
+        e = team.upload(da, (size_t)ra * es, a, (size_t)lda * es, (size_t)ra * es, ca, st);
+        if (e == cudaSuccess) e = team.upload(db, (size_t)rb * es, b, (size_t)ldb * es, (size_t)rb * es, cb, st);
     }
     if (e == cudaSuccess && beta != T(0))
-        e = cudaMemcpy2DAsync(dc, (size_t)m * es, c, (size_t)ldc * es, (size_t)m * es, n, cudaMemcpyHostToDevice, st);
+        e = team.upload(dc, (size_t)m * es, c, (size_t)ldc * es, (size_t)m * es, n, st);
     if (e == cudaSuccess) {
         GemmArgs<T> g{ta, tb, m, n, k, alpha, da, ra, db, rb, beta, dc, m};
         e = run_gemm(g, st, HostScratch{&cx});
@@ -338,7 +334,7 @@ void host_gemm(const char* routine, char ta, char tb, int m, int n, int k, T alp
         report_gpu_failure(routine);
         return;
     }
-    e = cudaMemcpy2DAsync(c, (size_t)ldc * es, dc, (size_t)m * es, (size_t)m * es, n, cudaMemcpyDeviceToHost, st);
+    e = team.download(c, (size_t)ldc * es, dc, (size_t)m * es, (size_t)m * es, n, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         cuda_status(e, "result copy");
@@ -467,14 +463,12 @@ void host_complex_gemm(const char* routine, char ta, char tb, int m, int n, int 
     T* da = static_cast<T*>(cx.stage_a.ptr);
     T* db = static_cast<T*>(cx.stage_b.ptr);
     T* dc = static_cast<T*>(cx.stage_c.ptr);
+    CopyTeam team(cx.slots, cx.device);
     if (!quick) {
-        e = cudaMemcpy2DAsync(da, (size_t)ra * es, a, (size_t)lda * es, (size_t)ra * es, ca, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess)
-            e = cudaMemcpy2DAsync(db, (size_t)rb * es, b, (size_t)ldb * es, (size_t)rb * es, cb, cudaMemcpyHostToDevice,
-                                  st);
+        e = team.upload(da, (size_t)ra * es, a, (size_t)lda * es, (size_t)ra * es, ca, st);
+        if (e == cudaSuccess) e = team.upload(db, (size_t)rb * es, b, (size_t)ldb * es, (size_t)rb * es, cb, st);
     }
-    if (e == cudaSuccess && !beta0)
-        e = cudaMemcpy2DAsync(dc, (size_t)m * es, c, (size_t)ldc * es, (size_t)m * es, n, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && !beta0) e = team.upload(dc, (size_t)m * es, c, (size_t)ldc * es, (size_t)m * es, n, st);
     if (e == cudaSuccess) {
         ComplexArgs<T> g{ta, tb, m, n, k, {alpha[0], alpha[1]}, da, ra, db, rb, {beta[0], beta[1]}, dc, m};
         e = run_complex(g, st, HostScratch{&cx});
@@ -485,7 +479,7 @@ void host_complex_gemm(const char* routine, char ta, char tb, int m, int n, int 
         report_gpu_failure(routine);
         return;
     }
-    e = cudaMemcpy2DAsync(c, (size_t)ldc * es, dc, (size_t)m * es, (size_t)m * es, n, cudaMemcpyDeviceToHost, st);
+    e = team.download(c, (size_t)ldc * es, dc, (size_t)m * es, (size_t)m * es, n, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         cuda_status(e, "result copy");

@@ -1,0 +1,222 @@
+// Staged copies of the host entry points.
+//
+// A pageable cudaMemcpy goes through the driver's own staging buffer on the
+// calling thread: 11.7 GB/s for dgemm_ 2048^3 (67 MB up, 34 MB down), a quarter
+// of the PCIe link and most of a call whose product takes 0.55 ms.  Here up to
+// eight host threads copy 512 KB chunks into pinned slots and enqueue each
+// chunk's device copy themselves; with two slots a thread fills one while the
+// other is on the link.  dgemm_ 2048^3 8.1 -> 4.0 ms a call, 1024^3 2.2 -> 1.4.
+// Page-locked memory and transfers under 2 MB (starting the threads would not
+// pay) keep cudaMemcpy2DAsync.
+#include "host_copy.h"
+
+#include <algorithm>
+#include <chrono>
+#include <cstring>
+#include <system_error>
+
+namespace zb {
+
+namespace {
+constexpr size_t kStagedMinBytes = size_t(2) << 20;
+}
+
+cudaError_t PinnedSlots::reserve() {
+    if (base) return cudaSuccess;
+    void* p = nullptr;
+    cudaError_t e = cudaHostAlloc(&p, 2 * kThreads * kSlotBytes, cudaHostAllocDefault);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return e;
+    }
+    base = static_cast<char*>(p);
+    for (cudaEvent_t& ev : done)
+        if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) {
+            cudaGetLastError();
+            release();
+            return e;
+        }
+    return cudaSuccess;
+}
+
+void PinnedSlots::release() {
+    for (cudaEvent_t& ev : done) {
+        if (ev) {
+            cudaEventSynchronize(ev);
+            cudaEventDestroy(ev);
+        }
+        ev = nullptr;
+    }
+    if (base) cudaFreeHost(base);
+    base = nullptr;
+}
+
+CopyTeam::~CopyTeam() {
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        quit_ = true;
+        posted_.store(-1, std::memory_order_release);
+    }
+    start_.notify_all();
+    for (std::thread& t : threads_) t.join();
+}
+
+// Whether this transfer goes through the slots; starts the threads the first time.
+bool CopyTeam::staged(const void* host, size_t width, size_t height) {
+    if (width * height < kStagedMinBytes) return false;
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (attr.type != cudaMemoryTypeUnregistered) return false;
+    const int want = std::min<int>(PinnedSlots::kThreads, (int)std::thread::hardware_concurrency() / 2);
+    if (want < 2 || slots_.reserve() != cudaSuccess) return false;
+    try {
+        while ((int)threads_.size() < want - 1) {
+            const int id = (int)threads_.size() + 1;
+            threads_.emplace_back([this, id] { loop(id); });
+        }
+    } catch (const std::system_error&) {  // no more threads: those that started, and this one, do the work
+    }
+    return true;
+}
+
+void CopyTeam::loop(int id) {
+    cudaSetDevice(device_);
+    long seen = 0;
+    for (;;) {
+        // the transfers of one call follow each other within microseconds: poll for the next
+        // one for a while before sleeping (a wake-up costs 50 to 100 us here)
+        const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(200);
+        while (posted_.load(std::memory_order_acquire) == seen && std::chrono::steady_clock::now() < until)
+            std::this_thread::yield();
+        {
+            std::unique_lock<std::mutex> lock(mu_);
+            start_.wait(lock, [&] { return quit_ || generation_ != seen; });
+            if (quit_) return;
+            seen = generation_;
+        }
+        work(id);
+        std::lock_guard<std::mutex> lock(mu_);
+        if (--busy_ == 0) finish_.notify_one();
+    }
+}
+
+// This thread's share of the current job: chunks claimed from a counter, alternating
+// between the thread's two slots.  A download's chunk is copied out of its slot while
+// the next one is on the link.
+void CopyTeam::work(int id) {
+    const Job& j = job_;
+    struct Chunk {
+        size_t col, cols, at, bytes;  // bytes at .. at + bytes of columns col .. col + cols
+    } held{};
+    int held_slot = -1, turn = 0;
+    auto fail = [&](cudaError_t e) {
+        int none = 0;
+        if (e != cudaSuccess) error_.compare_exchange_strong(none, (int)e);
+        return e != cudaSuccess;
+    };
+    auto rows = [&](const Chunk& c, char* slot, bool in) {
+        for (size_t q = 0; q < c.cols; ++q) {
+            char* h = j.host + (c.col + q) * j.hpitch + c.at;
+            if (in)
+                std::memcpy(slot + q * c.bytes, h, c.bytes);
+            else
+                std::memcpy(h, slot + q * c.bytes, c.bytes);
+        }
+    };
+    // slot <-> device: one run of bytes where the device columns are packed
+    auto link = [&](char* dst, size_t dp, const char* src, size_t sp, const Chunk& c, cudaMemcpyKind kind) {
+        if (c.cols == 1 || dp == sp) return cudaMemcpyAsync(dst, src, c.bytes * c.cols, kind, j.st);
+        return cudaMemcpy2DAsync(dst, dp, src, sp, c.bytes, c.cols, kind, j.st);
+    };
+    auto flush = [&]() {  // copy the held chunk of a download out
+        if (held_slot < 0) return;
+        if (!fail(cudaEventSynchronize(slots_.done[held_slot])))
+            rows(held, slots_.base + held_slot * PinnedSlots::kSlotBytes, false);
+        held_slot = -1;
+    };
+    for (;;) {
+        const size_t n = next_.fetch_add(1);
+        if (n >= j.chunks || error_.load()) break;
+        Chunk c;
+        if (j.pieces > 1) {
+            const size_t piece = PinnedSlots::kSlotBytes;
+            c = {n / j.pieces, 1, (n % j.pieces) * piece, 0};
+            c.bytes = std::min(piece, j.width - c.at);
+        } else {
+            c = {n * j.cols_per_chunk, 0, 0, j.width};
+            c.cols = std::min(j.cols_per_chunk, j.height - c.col);
+        }
+        const int s = 2 * id + (turn++ & 1);
+        char* slot = slots_.base + s * PinnedSlots::kSlotBytes;
+        char* dev = j.dev + c.col * j.dpitch + c.at;
+        if (fail(cudaEventSynchronize(slots_.done[s]))) break;  // the slot's last device copy
+        if (j.up) {
+            rows(c, slot, true);
+            if (fail(link(dev, j.dpitch, slot, c.bytes, c, cudaMemcpyHostToDevice))) break;
+            if (fail(cudaEventRecord(slots_.done[s], j.st))) break;
+        } else {
+            if (fail(link(slot, c.bytes, dev, j.dpitch, c, cudaMemcpyDeviceToHost))) break;
+            if (fail(cudaEventRecord(slots_.done[s], j.st))) break;
+            flush();
+            held = c;
+            held_slot = s;
+        }
+    }
+    flush();
+}
+
+cudaError_t CopyTeam::run(Job j) {
+    j.cols_per_chunk = std::max<size_t>(1, PinnedSlots::kSlotBytes / std::max<size_t>(1, j.width));
+    j.pieces = j.width > PinnedSlots::kSlotBytes ? (j.width + PinnedSlots::kSlotBytes - 1) / PinnedSlots::kSlotBytes : 1;
+    j.chunks = j.pieces > 1 ? j.height * j.pieces : (j.height + j.cols_per_chunk - 1) / j.cols_per_chunk;
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        job_ = j;
+        next_.store(0);
+        error_.store(0);
+        busy_ = (int)threads_.size();
+        posted_.store(++generation_, std::memory_order_release);
+    }
+    start_.notify_all();
+    work(0);
+    std::unique_lock<std::mutex> lock(mu_);
+    finish_.wait(lock, [&] { return busy_ == 0; });
+    return static_cast<cudaError_t>(error_.load());
+}
+
+cudaError_t CopyTeam::upload(void* dev, size_t dpitch, const void* host, size_t hpitch, size_t width, size_t height,
+                             cudaStream_t st) {
+    if (!staged(host, width, height))
+        return cudaMemcpy2DAsync(dev, dpitch, host, hpitch, width, height, cudaMemcpyHostToDevice, st);
+    Job j;
+    j.up = true;
+    j.host = static_cast<char*>(const_cast<void*>(host));
+    j.dev = static_cast<char*>(dev);
+    j.hpitch = hpitch;
+    j.dpitch = dpitch;
+    j.width = width;
+    j.height = height;
+    j.st = st;
+    return run(j);
+}
+
+cudaError_t CopyTeam::download(void* host, size_t hpitch, const void* dev, size_t dpitch, size_t width, size_t height,
+                               cudaStream_t st) {
+    if (!staged(host, width, height))
+        return cudaMemcpy2DAsync(host, hpitch, dev, dpitch, width, height, cudaMemcpyDeviceToHost, st);
+    Job j;
+    j.up = false;
+    j.host = static_cast<char*>(host);
+    j.dev = static_cast<char*>(const_cast<void*>(dev));
+    j.hpitch = hpitch;
+    j.dpitch = dpitch;
+    j.width = width;
+    j.height = height;
+    j.st = st;
+    return run(j);
+}
+
+}  // namespace zb

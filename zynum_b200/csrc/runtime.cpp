@@ -143,6 +143,7 @@ void Context::shutdown() {
     stream_work.clear();
     cudaStreamSynchronize(stream_in);
     cudaStreamSynchronize(stream_out);
+    slots.release();
     cudaStreamDestroy(stream);
     cudaStreamDestroy(stream_in);
     cudaStreamDestroy(stream_out);

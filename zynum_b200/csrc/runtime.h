@@ -19,6 +19,8 @@
 
 #include <cuda_runtime.h>
 
+#include "host_copy.h"
+
 namespace zb {
 
 enum DgemmMethod : int { METHOD_NATIVE = 0, METHOD_OZAKI = 1, METHOD_AUTO = 2 };
@@ -60,6 +62,7 @@ struct Context {
     cudaStream_t stream_in = nullptr, stream_out = nullptr;
     std::recursive_mutex mutex;     // host entry points are callable from any thread
     DeviceBuffer stage_a, stage_b, stage_c;
+    PinnedSlots slots;  // staging of pageable host matrices
     DeviceBuffer work;  // scratch of the host entry points (split-K partials, slices)
     // Scratch of the device entry points, one per caller stream so that calls
     // on different streams never share scratch memory.
