@@ -203,6 +203,168 @@ dgemm_dmma_kernel(int M, int N, int K, int k_chunk, double alpha, const double* 
     }
 }
 
+// ------------------------------------------------- 64 x 64 tiles in clusters
+// Small products: a 64 x 64 tile per cluster, K split over its CTAs (blockIdx.z), each of
+// which leaves its partial tile in shared memory and sums 64 / splits columns of all of
+// them through distributed shared memory, in rank order (deterministic).  Bound: launch
+// and memory latency.  Against 64 x 64 tiles with partials in a workspace and a reduction
+// kernel this saves the second launch (256^3 called back to back: 12.4 -> 9.9 us, bound by
+// the host's launches; on the device 6.5 / 6.6) and the partials' round trip through L2
+// (512^3: 16.0 -> 15.3 us, 128^3: 6.6 -> 5.1, 255^3 with odd leading dimensions 9.8 -> 7.1).
+// Eight warps of 32 x 16, fragments double-buffered in registers.
+constexpr int kCM = 64, kCN = 64, kCThreads = 256, kCStages = 4;
+constexpr int kCPitch = kCM + 2;  // partial tile [col][row]: 16-byte rows, conflict-free fragment stores
+
+ZB_DEVICE void ld_cluster_f64x2(uint32_t addr, double& x, double& y) {
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];\n" : "=d"(x), "=d"(y) : "r"(addr) : "memory");
+}
+
+template <bool A_KFAST, bool B_KFAST, int VEC>
+__global__ void __launch_bounds__(kCThreads, 2)
+dgemm_cluster_kernel(int M, int N, int K, int k_chunk, double alpha, const double* __restrict__ A, long lda,
+                     const double* __restrict__ B, long ldb, double beta, double* __restrict__ C, long ldc, int tri) {
+    constexpr int A_ROWS = A_KFAST ? kCM : kBK, A_COLS = A_KFAST ? kBK : kCM, A_PITCH = A_COLS + 4;
+    constexpr int B_ROWS = B_KFAST ? kCN : kBK, B_COLS = B_KFAST ? kBK : kCN, B_PITCH = B_COLS + 4;
+    constexpr int A_STAGE = A_ROWS * A_PITCH, B_STAGE = B_ROWS * B_PITCH;
+    constexpr int STAGES = kCStages, MI = 2, NI = 2;  // warp tile 32 x 16, warps 2 x 4
+
+    extern __shared__ __align__(128) double smem[];
+    double* As = smem;
+    double* Bs = smem + STAGES * A_STAGE;
+
+    const int m0 = blockIdx.x * kCM, n0 = blockIdx.y * kCN;
+    // triangle mode: the whole cluster skips a tile that holds no element of the stored triangle
+    if ((tri == 1 && m0 > n0 + kCN - 1) || (tri == 2 && m0 + kCM - 1 < n0)) return;
+    const int splits = gridDim.z, rank = blockIdx.z;  // the cluster spans gridDim.z
+    const int kb = rank * k_chunk, ke = min(K, kb + k_chunk);
+    const int KT = max(0, (ke - kb + kBK - 1) / kBK);
+    grid_dependency_wait();
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int wm = (warp >> 2) * 32, wn = (warp & 3) * 16;
+    const int g = lane >> 2, t = lane & 3;
+    double acc[MI][NI][4];
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[i][j][v] = 0.0;
+
+    auto load_stage = [&](int stage, int kt) {
+        const int k0 = kb + kt * kBK;
+        if (A_KFAST)
+            load_tile<A_ROWS, A_COLS, A_PITCH, VEC, kCThreads>(As + stage * A_STAGE, A, lda, m0, k0, M, ke);
+        else
+            load_tile<A_ROWS, A_COLS, A_PITCH, VEC, kCThreads>(As + stage * A_STAGE, A, lda, k0, m0, ke, M);
+        if (B_KFAST)
+            load_tile<B_ROWS, B_COLS, B_PITCH, VEC, kCThreads>(Bs + stage * B_STAGE, B, ldb, n0, k0, N, ke);
+        else
+            load_tile<B_ROWS, B_COLS, B_PITCH, VEC, kCThreads>(Bs + stage * B_STAGE, B, ldb, k0, n0, ke, N);
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (s < KT) load_stage(s, s);
+        cp_async_commit();
+    }
+    // Fragments are double-buffered in registers: the loads of step ks + 8 (of the
+    // next slice in a slice's last step) are issued before the products of step ks.
+    double af[2][MI][4], bf[2][NI][2];
+    auto load_frag = [&](int buf, int st, int ks) {
+        const double* as = As + st * A_STAGE;
+        const double* bs = Bs + st * B_STAGE;
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                const int rr = wm + i * 16 + g + 8 * (v & 1), kk = ks + t + 4 * (v >> 1);
+                af[buf][i][v] = A_KFAST ? as[rr * A_PITCH + kk] : as[kk * A_PITCH + rr];
+            }
+#pragma unroll
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int cc = wn + j * 8 + g, kk = ks + t + 4 * v;
+                bf[buf][j][v] = B_KFAST ? bs[cc * B_PITCH + kk] : bs[kk * B_PITCH + cc];
+            }
+    };
+    static_assert(kBK == 16, "two k8 steps per slice");
+    int stage = 0;
+    cp_async_wait<STAGES - 2>();
+    __syncthreads();
+    load_frag(0, 0, 0);
+    for (int kt = 0; kt < KT; ++kt) {
+        load_frag(1, stage, 8);
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NI; ++j) dmma_16x8x8(acc[i][j], af[0][i], bf[0][j]);
+        {
+            const int nk = kt + STAGES - 1;
+            if (nk < KT) load_stage(stage == 0 ? STAGES - 1 : stage - 1, nk);
+            cp_async_commit();
+        }
+        if (++stage == STAGES) stage = 0;
+        if (kt + 1 < KT) {
+            cp_async_wait<STAGES - 2>();
+            __syncthreads();
+            load_frag(0, stage, 0);
+        }
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NI; ++j) dmma_16x8x8(acc[i][j], af[1][i], bf[1][j]);
+    }
+    cp_async_wait<0>();
+    __syncthreads();  // the ring is reused for the partial tile
+
+    double* P = smem;
+#pragma unroll
+    for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+                P[(wn + j * 8 + 2 * t + (v & 1)) * kCPitch + wm + i * 16 + g + 8 * (v >> 1)] = acc[i][j][v];
+    if (splits > 1)
+        cluster_sync();
+    else
+        __syncthreads();
+    // CTA `rank` sums, in rank order, and writes columns rank * 64 / splits ..
+    const int cols = kCN / splits, c_first = rank * cols;
+    for (int q = threadIdx.x; q < cols * (kCM / 2); q += kCThreads) {
+        const int r = (q % (kCM / 2)) * 2, c = c_first + q / (kCM / 2);
+        const int row = m0 + r, col = n0 + c;
+        if (row >= M || col >= N) continue;
+        const uint32_t at = smem_u32(P + c * kCPitch + r);
+        double x0 = 0.0, x1 = 0.0;
+        if (splits == 1) {
+            x0 = P[c * kCPitch + r];
+            x1 = P[c * kCPitch + r + 1];
+        } else {
+            for (int z = 0; z < splits; ++z) {
+                double y0, y1;
+                ld_cluster_f64x2(mapa_shared(at, z), y0, y1);
+                x0 += y0;
+                x1 += y1;
+            }
+        }
+        double* cp = C + (long)col * ldc + row;
+        const bool in0 = tri == 0 || (tri == 1 ? row <= col : row >= col);
+        const bool in1 = row + 1 < M && (tri == 0 || (tri == 1 ? row + 1 <= col : row + 1 >= col));
+        x0 *= alpha;
+        x1 *= alpha;
+        if (beta != 0.0) {
+            const double c0 = in0 ? cp[0] : 0.0, c1 = in1 ? cp[1] : 0.0;
+            x0 = fma(beta, c0, x0);
+            x1 = fma(beta, c1, x1);
+        }
+        if (in0) cp[0] = x0;
+        if (in1) cp[1] = x1;
+    }
+    if (splits > 1) cluster_sync();  // no CTA leaves while its partial tile may be read
+}
+
 __global__ void dgemm_splitk_reduce(int M, int N, int splits, const double* __restrict__ W, double alpha, double beta,
                                     double* __restrict__ C, long ldc, int tri) {
     grid_dependency_wait();  // launched during the tail of the product that writes W
@@ -259,6 +421,35 @@ cudaError_t splitk_reduce(const GemmArgsF64& g, int used_splits, double* workspa
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
+template <bool AK, bool BKF, int VEC>
+cudaError_t launch_cluster(const GemmArgsF64& g, int splits, cudaStream_t st) {
+    constexpr int A_STAGE = AK ? kCM * (kBK + 4) : kBK * (kCM + 4), B_STAGE = BKF ? kCN * (kBK + 4) : kBK * (kCN + 4);
+    constexpr size_t SMEM = (size_t)kCStages * (A_STAGE + B_STAGE) * sizeof(double);
+    static_assert(SMEM >= (size_t)kCN * kCPitch * sizeof(double), "the partial tile reuses the ring");
+    auto kern = dgemm_cluster_kernel<AK, BKF, VEC>;
+    cudaError_t e = ensure_dynamic_smem(kern, (int)SMEM);
+    if (e != cudaSuccess) return e;
+    int k_chunk = (g.k + splits - 1) / splits;
+    k_chunk = (k_chunk + kBK - 1) / kBK * kBK;
+    const dim3 grid((g.m + kCM - 1) / kCM, (g.n + kCN - 1) / kCN, splits);
+    prof_begin(st);
+    e = launch_dependent_cluster(kern, grid, dim3(kCThreads), SMEM, st, dim3(1, 1, splits), g.m, g.n, g.k, k_chunk,
+                                 g.alpha, g.a, g.lda, g.b, g.ldb, g.beta, g.c, g.ldc, g.tri);
+    count_launch();
+    prof_end(st);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+cudaError_t run_cluster(const GemmArgsF64& g, int vec, int splits, cudaStream_t st) {
+    const bool ak = g.transa != 'N', bk = g.transb == 'N';
+#define ZB_CASE(AK, BKF, V) \
+    if (ak == AK && bk == BKF && vec == V) return launch_cluster<AK, BKF, V>(g, splits, st);
+    ZB_CASE(false, false, 1) ZB_CASE(false, true, 1) ZB_CASE(true, false, 1) ZB_CASE(true, true, 1)
+    ZB_CASE(false, false, 2) ZB_CASE(false, true, 2) ZB_CASE(true, false, 2) ZB_CASE(true, true, 2)
+#undef ZB_CASE
+    return cudaErrorInvalidValue;
+}
+
 template <int BM, int BN, int WM, int WN, int STAGES, int BK = kBK>
 cudaError_t run_tiles(const GemmArgsF64& g, int vec, int used_splits, int k_chunk, double* workspace,
                       cudaStream_t st) {
@@ -306,6 +497,16 @@ static int ws_cluster(const GemmArgsF64& g, const GemmPlan& plan) {
     return r64 < 0.98 * r128 ? 1 : 0;
 }
 
+// Cluster size with which a planned small product runs on the 64 x 64 cluster tiles
+// (dgemm_cluster_kernel: one launch, none of the plan's workspace); 0: it does not.
+static int small_cluster(const GemmArgsF64& g, const GemmPlan& plan) {
+    // up to two CTAs per SM, and no fewer K ranges than the workspace route has (which splits
+    // down to 64-deep slices: 256 x 256 x 1024 takes it 9.6 us, a cluster of 8 15.1)
+    const long t64 = (long)((g.m + 63) / 64) * ((g.n + 63) / 64);
+    if (!plan.automatic || plan.tile != TILE_64x64 || plan.splits < 2 || 4 * t64 > 2 * 148) return 0;
+    return g.k <= 256 || plan.splits == 4 ? 4 : 0;
+}
+
 int dgemm_native_used_splits(const GemmArgsF64& g, const GemmPlan& plan) {
     const int splits = plan.splits < 1 ? 1 : plan.splits;
     if (plan.tile == TILE_GEMV && gemv_applies(g.m, g.n, g.k, g.tri)) return gemv_used_splits(g.k, splits);
@@ -334,6 +535,7 @@ cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* wor
     k_chunk = (k_chunk + kBK - 1) / kBK * kBK;
     const int used = (g.k + k_chunk - 1) / k_chunk;
     if (const int ws = ws_cluster(g, plan)) return dgemm_ws(g, ws, st);
+    if (const int c = small_cluster(g, plan)) return run_cluster(g, vec, c, st);
     switch (plan.tile) {
         case TILE_128x64:
             return run_tiles<128, 64, 64, 32, 4>(g, vec, used, k_chunk, workspace, st);
