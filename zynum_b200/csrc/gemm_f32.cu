@@ -38,6 +38,10 @@ template <>
 struct Cfg<128> {
     static constexpr int BK = 16, STAGES = 5, MINB = 2;
 };
+template <>
+struct Cfg<64> {
+    static constexpr int BK = 16, STAGES = 4, MINB = 3;
+};
 __host__ __device__ constexpr int pitch(int width) { return width + 4; }  // floats per shared row ([k][mn], mn fast)
 
 // Copy a BK x WIDTH tile (rows k, columns mn) into shared memory.
@@ -122,23 +126,14 @@ ZB_DEVICE void unpack_f32x2(uint64_t v, float& x, float& y) {
 // {64 q + tx*4 + j}, q < BN / 64; a warp covers 4 ty x 8 tx, so each float4
 // fragment load touches 4 (A) or 8 (B) distinct 16-byte words: one
 // shared-memory wavefront.
-template <bool A_MNFAST, bool B_MNFAST, int VEC, bool PARTIAL, int BN>
-__global__ void __launch_bounds__(kThreads, Cfg<BN>::MINB)
-sgemm_ffma_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __restrict__ A, long lda,
-                  const float* __restrict__ B, long ldb, float beta, float* __restrict__ C, long ldc,
-                  float* __restrict__ W, int tri) {
+template <bool A_MNFAST, bool B_MNFAST, int VEC, int BN>
+ZB_DEVICE void sgemm_products(float (&acc)[8][BN / 16], float* smf, int M, int N, int m0, int n0, int kb, int ke,
+                              const float* __restrict__ A, long lda, const float* __restrict__ B, long ldb) {
     constexpr int BK = Cfg<BN>::BK, STAGES = Cfg<BN>::STAGES, JN = BN / 16, PA = pitch(kBM), PB = pitch(BN);
-    extern __shared__ __align__(128) float smf[];
     float* As = smf;
     float* Bs = smf + STAGES * BK * PA;
     using LA = TileLoader<A_MNFAST, (A_MNFAST ? VEC : 1), kBM, BK>;
     using LB = TileLoader<B_MNFAST, (B_MNFAST ? VEC : 1), BN, BK>;
-
-    const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
-    // triangle mode: skip tiles that hold no element of the stored triangle
-    if ((tri == 1 && m0 > n0 + BN - 1) || (tri == 2 && m0 + kBM - 1 < n0)) return;
-    const int kb = blockIdx.z * k_chunk;
-    const int ke = min(K, kb + k_chunk);
     const int KT = (ke - kb + BK - 1) / BK;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);
@@ -198,11 +193,29 @@ sgemm_ffma_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __
         }
     }
     cp_async_wait<0>();
-    float acc[8][JN];
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
         for (int j = 0; j < JN; ++j) unpack_f32x2(acc2[p][j], acc[2 * p][j], acc[2 * p + 1][j]);
+}
+
+template <bool A_MNFAST, bool B_MNFAST, int VEC, bool PARTIAL, int BN>
+__global__ void __launch_bounds__(kThreads, Cfg<BN>::MINB)
+sgemm_ffma_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __restrict__ A, long lda,
+                  const float* __restrict__ B, long ldb, float beta, float* __restrict__ C, long ldc,
+                  float* __restrict__ W, int tri) {
+    constexpr int JN = BN / 16;
+    extern __shared__ __align__(128) float smf[];
+
+    const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * BN;
+    // triangle mode: skip tiles that hold no element of the stored triangle
+    if ((tri == 1 && m0 > n0 + BN - 1) || (tri == 2 && m0 + kBM - 1 < n0)) return;
+    const int kb = blockIdx.z * k_chunk;
+    const int ke = min(K, kb + k_chunk);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);
+    float acc[8][JN];
+    sgemm_products<A_MNFAST, B_MNFAST, VEC, BN>(acc, smf, M, N, m0, n0, kb, ke, A, lda, B, ldb);
 
     // Rows ty*4 .. ty*4+3 of one column are contiguous in column-major C:
     // one 16-byte access when the destination allows it.
@@ -256,6 +269,70 @@ sgemm_ffma_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __
     }
 }
 
+// Few output tiles: 128 x 64 tiles with K split over a cluster of gridDim.z CTAs (1, 2, 4
+// or 8).  Each leaves its partial tile in shared memory and sums 64 / splits columns of all
+// of them through distributed shared memory in rank order: no workspace, no second launch.
+// Bound: latency and the share of the SMs a small product can use; 128 x 128 tiles with
+// slices of at least 256 left most of them idle (512^3: 32 CTAs).  512^3 34.6 -> 12.3 us,
+// 256^3 31.0 -> 6.3, 128^3 15.8 -> 5.6, 64 x 2000 x 100 TT 15.8 -> 8.0.
+constexpr int kCN = 64, kCPitch = kBM + 4;
+
+template <bool A_MNFAST, bool B_MNFAST, int VEC>
+__global__ void __launch_bounds__(kThreads, Cfg<kCN>::MINB)
+sgemm_cluster_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __restrict__ A, long lda,
+                     const float* __restrict__ B, long ldb, float beta, float* __restrict__ C, long ldc, int tri) {
+    constexpr int JN = kCN / 16;
+    extern __shared__ __align__(128) float smf[];
+    const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * kCN;
+    // triangle mode: the whole cluster skips a tile that holds no element of the stored triangle
+    if ((tri == 1 && m0 > n0 + kCN - 1) || (tri == 2 && m0 + kBM - 1 < n0)) return;
+    const int splits = gridDim.z, rank = blockIdx.z;
+    const int kb = min(K, rank * k_chunk), ke = min(K, kb + k_chunk);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);
+    float acc[8][JN];
+    sgemm_products<A_MNFAST, B_MNFAST, VEC, kCN>(acc, smf, M, N, m0, n0, kb, ke, A, lda, B, ldb);
+    __syncthreads();  // the ring becomes the partial tile [column][row]
+#pragma unroll
+    for (int j = 0; j < JN; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            *reinterpret_cast<float4*>(smf + (tx * 4 + j) * kCPitch + h * 64 + ty * 4) =
+                make_float4(acc[4 * h][j], acc[4 * h + 1][j], acc[4 * h + 2][j], acc[4 * h + 3][j]);
+    if (splits > 1)
+        cluster_sync();
+    else
+        __syncthreads();
+    const int cols = kCN / splits;
+    for (int q = threadIdx.x; q < cols * (kBM / 4); q += kThreads) {
+        const int r = (q % (kBM / 4)) * 4, c = rank * cols + q / (kBM / 4);
+        const int row = m0 + r, col = n0 + c;
+        if (row >= M || col >= N) continue;
+        const uint32_t at = smem_u32(smf + c * kCPitch + r);
+        float x[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int z = 0; z < splits; ++z) {
+            float4 y;
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];\n"
+                         : "=f"(y.x), "=f"(y.y), "=f"(y.z), "=f"(y.w)
+                         : "r"(mapa_shared(at, z))
+                         : "memory");
+            x[0] += y.x;
+            x[1] += y.y;
+            x[2] += y.z;
+            x[3] += y.w;
+        }
+        float* cp = C + (long)col * ldc + row;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (row + i >= M || (tri == 1 ? row + i > col : (tri == 2 && row + i < col))) continue;
+            float out = alpha * x[i];
+            if (beta != 0.f) out = fmaf(beta, cp[i], out);
+            cp[i] = out;
+        }
+    }
+    if (splits > 1) cluster_sync();  // no CTA leaves while its partial tile may be read
+}
+
 __global__ void sgemm_splitk_reduce(int M, int N, int splits, const float* __restrict__ W, float alpha, float beta,
                                     float* __restrict__ C, long ldc, int tri) {
     long total = (long)M * N;
@@ -285,6 +362,57 @@ cudaError_t launch_f32(const GemmArgsF32& g, int splits, int k_chunk, float* W, 
     count_launch();
     prof_end(st);
     return cudaGetLastError();
+}
+
+template <bool AM, bool BM_, int VEC>
+cudaError_t launch_cluster_f32(const GemmArgsF32& g, int splits, cudaStream_t st) {
+    constexpr size_t SMEM = (size_t)Cfg<kCN>::STAGES * Cfg<kCN>::BK * (pitch(kBM) + pitch(kCN)) * sizeof(float);
+    static_assert(SMEM >= (size_t)kCN * kCPitch * sizeof(float), "the partial tile reuses the ring");
+    auto kern = sgemm_cluster_kernel<AM, BM_, VEC>;
+    cudaError_t e = ensure_dynamic_smem(kern, (int)SMEM);
+    if (e != cudaSuccess) return e;
+    const int k_chunk = ((g.k + splits - 1) / splits + 15) / 16 * 16;
+    const dim3 grid((g.m + kBM - 1) / kBM, (g.n + kCN - 1) / kCN, splits);
+    prof_begin(st);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = splits;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kern, g.m, g.n, g.k, k_chunk, g.alpha, g.a, g.lda, g.b, g.ldb, g.beta, g.c, g.ldc,
+                           g.tri);
+    count_launch();
+    prof_end(st);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+// Cluster size of the 128 x 64 cluster tiles for a product planned with `splits` K ranges of
+// 128 x 128 tiles; 0: it keeps the plan.  The largest cluster with at most one CTA per SM and
+// 16-deep ranges, where its CTAs then have less to do than the plan's: (K / c) x 64 columns
+// against (K / splits) x 128 (1024^3: c = 1 against two K ranges, 65 against 61 us, keeps the plan;
+// 300 x 300 x 4000, c = 8 against 15: 36.9 / 37.1; 256 x 256 x 262144, c = 8 against 37, keeps it).
+int cluster_splits(const GemmArgsF32& g, int splits) {
+    const long t = (long)((g.m + kBM - 1) / kBM) * ((g.n + kCN - 1) / kCN);
+    for (int c = 8; c >= 1; c /= 2)
+        if (c * t <= 148 && (c == 1 || g.k >= 16 * c)) return 2 * c > splits ? c : 0;
+    return 0;
+}
+
+cudaError_t dispatch_cluster_f32(const GemmArgsF32& g, int vec, int splits, cudaStream_t st) {
+    const bool am = g.transa == 'N', bm = g.transb != 'N';
+#define ZB_CASE(AM, BMF, V) \
+    if (am == AM && bm == BMF && vec == V) return launch_cluster_f32<AM, BMF, V>(g, splits, st);
+    ZB_CASE(false, true, 1) ZB_CASE(true, false, 1) ZB_CASE(true, true, 1)
+    ZB_CASE(false, true, 4) ZB_CASE(true, false, 4) ZB_CASE(true, true, 4)
+#undef ZB_CASE
+    return launch_cluster_f32<false, false, 1>(g, splits, st);
 }
 
 template <bool PARTIAL>
@@ -423,6 +551,7 @@ cudaError_t sgemm_native(const GemmArgsF32& g_in, const GemmPlan& plan, float* w
     if (g.transb != 'N') aligned = aligned && (reinterpret_cast<uintptr_t>(g.b) % 16 == 0) && (g.ldb % 4 == 0);
     const int vec = aligned ? 4 : 1;
     const int splits = plan.splits < 1 ? 1 : plan.splits;
+    if (const int c = cluster_splits(g, splits)) return dispatch_cluster_f32(g, vec, c, st);
     int k_chunk = (g.k + splits - 1) / splits;
     k_chunk = (k_chunk + 31) / 32 * 32;  // a multiple of every BK
     const int used = (g.k + k_chunk - 1) / k_chunk;
