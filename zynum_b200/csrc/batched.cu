@@ -14,10 +14,11 @@
 // Operands are staged with cp.async (8- / 4-byte copies: per-problem leading
 // dimensions need not be aligned).
 //
-// TRSM (left side): one CTA solves one whole problem B := alpha op(A)^-1 B:
-// for every 64-row diagonal block, substitution on the block held in shared
-// memory, then the rank-64 update of the rows below (above) it with the
-// solved rows kept in shared memory.
+// TRSM (left side), B := alpha op(A)^-1 B: FP64 left-looking, one CTA per 32
+// right-hand sides of a problem; FP32 right-looking, one CTA per problem: for
+// every 64-row diagonal block, substitution on the block held in shared memory,
+// then the rank-64 update of the rows below (above) it with the solved rows
+// kept in shared memory.
 #include <algorithm>
 
 #include "batched.h"
@@ -460,8 +461,8 @@ ZB_DEVICE void substitute_rhs(T (*X)[kPP], const T (*D)[kTP], const T* dinv, int
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 2)
-trsm_batched_kernel(const int* __restrict__ order, int count, int* __restrict__ next, const int* __restrict__ dims, char uplo, char trans,
-                    char diag, T alpha, const T* const* __restrict__ a, const int* __restrict__ lda,
+trsm_batched_kernel(const int2* __restrict__ items, int count, int* __restrict__ next, const int* __restrict__ dims,
+                    char uplo, char trans, char diag, T alpha, const T* const* __restrict__ a, const int* __restrict__ lda,
                     T* const* __restrict__ b, const int* __restrict__ ldb) {
     extern __shared__ __align__(16) unsigned char trsm_smem[];
     // Two 64 x kPP buffers: the diagonal block D (pitch kTP) during the
@@ -479,7 +480,7 @@ trsm_batched_kernel(const int* __restrict__ order, int count, int* __restrict__ 
     Claim cl{next, claim_slot};
     for (int w = cl.first(); w < count; w = cl.advance()) {
         cl.prefetch();
-        const int q = order[w];
+        const int q = items[w].x;  // whole problems
         const int n = dims[2 * q], r = dims[2 * q + 1];
         const T* A = a[q];
         T* B = b[q];
@@ -634,149 +635,252 @@ trsm_batched_kernel(const int* __restrict__ order, int count, int* __restrict__ 
     }
 }
 
-// FP64 left-looking solver, one CTA per problem (left side, r <= 64): for each
-// 64-row block in solve order, acc = sum over the solved blocks j of
-// op(A)[block, j] X_j streams 32-deep K chunks of op(A) and of the solved rows
-// X (read back from B) through a two-stage cp.async ring into 16 x 8 DMMA tiles
-// held in registers (warp w: row tile w % 4, column tiles 4 (w / 4) .. +3);
-// then X_block = B_block - acc is solved in shared memory by a warp-synchronous
-// substitution (each warp carries only the right-hand sides it has) and
-// written back to B once.  The diagonal block's copy is in flight during the
-// products.
-constexpr int kLlK = 32;                          // K chunk
-constexpr int kLlPitch = kTB + 4;                 // 68: [k][row] and [k][col] tiles
-constexpr int kLlStage = 2 * kLlK * kLlPitch;     // A chunk + X chunk, in doubles
-constexpr int kLlRing = 2 * kLlStage;             // two stages (also holds the 64 x 68 solve block)
+// FP64 left-looking solver, one CTA per work item: up to kTrsmCols right-hand sides of one
+// problem (left side).  For each 64-row block in solve order, acc = sum over the solved
+// blocks j of op(A)[block, j] X_j streams 16-deep K chunks of op(A) and of the solved rows
+// X (read back from B) through a three-stage cp.async ring into 16 x 8 DMMA tiles held in
+// registers: warp w takes row tile w % 4 and all column tiles, for the first (w < 4) or the
+// second eight k of the chunk.  X_block = B_block - acc is then solved in shared memory by a
+// warp-synchronous substitution (each warp carries only the right-hand sides it has) and
+// written back to B once.  The diagonal block's copy is in flight during the products, the
+// next block's first chunk during the substitution.
+//
+// Bound: latency, per 64-row block about 3 us to issue the copies, 0.8 us per chunk, 4 to
+// form X and 6.5 for the substitution; op(A) once through HBM is a quarter of the time.  So
+// the split is for more independent blocks per SM and shorter chains: items of 32 columns
+// (a problem with 64 is two items and its chain half as long), the triangle packed into
+// 16.6 KB and a ring of 41 KB for three CTAs per SM.  5,000 problems (n 16..1024, 1..64
+// right-hand sides) 1.81 -> 1.45 ms, 1,800 of them 1.40 -> 0.98; with two 32-deep stages
+// and whole problems on two CTAs before.  A fourth stage is slower (1.58 ms: it leaves L1 too
+// little), two stages or no chunk ahead 1.48 / 1.42 (the latter 3 % slower on small batches).
+constexpr int kLlK = 16;                               // K chunk
+constexpr int kLlStages = 3;
+constexpr int kLlPA = kTB + 4;                         // op(A) chunk [k][row]
+constexpr int kLlPX = kLlK + 4;                        // X chunk [column][k]: copies and fragment loads conflict-free
+constexpr int kLlStage = kLlK * kLlPA + kTrsmCols * kLlPX;
+constexpr int kLlRing = kLlStages * kLlStage;
+constexpr int kLlAhead = 1;                            // chunks of the next block loaded before the substitution
+constexpr int kLlXP = kTrsmCols + 4;
+constexpr int kLlTri = 32 * (kTB + 1);                 // packed triangle of the diagonal block
+static_assert(kTB * kLlXP <= (kLlStages - kLlAhead) * kLlStage, "the solve block reuses the last stages");
 
-__global__ void __launch_bounds__(kThreads, 2)
-trsm_batched_ll_f64(const int* __restrict__ order, int count, int* __restrict__ next, const int* __restrict__ dims, char uplo, char trans,
-                    char diag, double alpha, const double* const* __restrict__ a, const int* __restrict__ lda,
-                    double* const* __restrict__ b, const int* __restrict__ ldb) {
+// Position of element (r, c), c <= r, of a packed 64 x 64 lower triangle: rows r and 63 - r
+// share one row of 65.  A lane per row reads any column without bank conflicts.
+ZB_DEVICE int tri_at(int r, int c) { return r >= 32 ? (kTB - 1 - r) * (kTB + 1) + c : r * (kTB + 1) + kTB - c; }
+
+// One half of the substitution as substitute_half, on the packed triangle in solve order
+// (row / column s of D is row s of a lower block, its last row minus s for an upper one, so
+// that every solve is a lower one) with its columns scaled by 1 / D[s][s]: a row's unscaled
+// final value is broadcast, so that a step is one shuffle and one FMA deep.  Lane l owns
+// solve rows l and l + 32.
+template <int CM, int HI>
+ZB_DEVICE void substitute_tri(double (&x)[2][CM], const double* D, int sz) {
+    const int lane = threadIdx.x & 31;
+    const int lo = 32 * HI, hi = min(sz, lo + 32);
+    for (int i = lo; i < hi; ++i) {
+        double xi[CM];
+#pragma unroll
+        for (int c = 0; c < CM; ++c) xi[c] = __shfl_sync(0xffffffffu, x[HI][c], i & 31);
+        if (HI == 0) {  // every row of the second half
+            const double d = D[tri_at(lane + 32, i)];
+#pragma unroll
+            for (int c = 0; c < CM; ++c) x[1][c] = fma(-d, xi[c], x[1][c]);
+        }
+        const int p = lane + 32 * HI;
+        if (p > i) {
+            const double d = D[tri_at(p, i)];
+#pragma unroll
+            for (int c = 0; c < CM; ++c) x[HI][c] = fma(-d, xi[c], x[HI][c]);
+        }
+    }
+}
+
+// X: solve rows x columns; warp w carries columns w + 8 c, c < CM.
+template <int CM>
+ZB_DEVICE void substitute_packed(double (*X)[kLlXP], const double* D, const double* dinv, int sz) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double x[2][CM];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int c = 0; c < CM; ++c) x[h][c] = X[lane + 32 * h][warp + 8 * c];
+    substitute_tri<CM, 0>(x, D, sz);
+    if (sz > 32) substitute_tri<CM, 1>(x, D, sz);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const double s = dinv[lane + 32 * h];
+#pragma unroll
+        for (int c = 0; c < CM; ++c) X[lane + 32 * h][warp + 8 * c] = x[h][c] * s;
+    }
+}
+
+__global__ void __launch_bounds__(kThreads, kTrsmCtasPerSm)
+trsm_batched_ll_f64(const int2* __restrict__ items, int count, int* __restrict__ next, const int* __restrict__ dims,
+                    char uplo, char trans, char diag, double alpha, const double* const* __restrict__ a,
+                    const int* __restrict__ lda, double* const* __restrict__ b, const int* __restrict__ ldb) {
     extern __shared__ __align__(16) unsigned char ll_smem[];
     double* ring = reinterpret_cast<double*>(ll_smem);
-    double(*X)[kPP] = reinterpret_cast<double(*)[kPP]>(ring);  // solve block, after the products
-    double(*D)[kTP] = reinterpret_cast<double(*)[kTP]>(ring + kLlRing);
-    double* dinv = ring + kLlRing + kTB * kTP;
+    double(*X)[kLlXP] = reinterpret_cast<double(*)[kLlXP]>(ring + kLlAhead * kLlStage);  // solve block, after the products
+    double* D = ring + kLlRing;
+    double* dinv = D + kLlTri;
     const bool upper = (trans == 'N' && uplo == 'U') || (trans != 'N' && uplo == 'L');
     const bool unit = diag == 'U';
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, g = lane >> 2, tq = lane & 3;
-    const int rt = warp & 3, ct0 = (warp >> 2) * 4;
+    const int rt = warp & 3, kh = warp >> 2;
     __shared__ int claim_slot[2];
     Claim cl{next, claim_slot};
     for (int w = cl.first(); w < count; w = cl.advance()) {
         cl.prefetch();
-        const int q = order[w];
-        const int n = dims[2 * q], r = dims[2 * q + 1];
+        const int2 item = items[w];
+        const int q = item.x, n = dims[2 * q], r = min(kTrsmCols, dims[2 * q + 1] - item.y);
         const double* A = a[q];
-        double* B = b[q];
         const long la = lda[q], lb = ldb[q];
-        if (alpha != 1.0)  // eight loads in flight per thread before their stores
-            for (long e0 = t; e0 < (long)n * r; e0 += 8L * kThreads) {
-                double v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const long e = e0 + (long)u * kThreads;
-                    v[u] = e < (long)n * r ? B[(e % n) + (e / n) * lb] : 0.0;
-                }
-#pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const long e = e0 + (long)u * kThreads;
-                    if (e < (long)n * r) B[(e % n) + (e / n) * lb] = alpha * v[u];
-                }
-            }
-        __syncthreads();
+        double* B = b[q] + (long)item.y * lb;
+        const long rs = trans == 'N' ? 1 : la, ks = trans == 'N' ? la : 1;  // strides of a row / column of op(A)
         const int nblk = (n + kTB - 1) / kTB, nct = (r + 7) / 8;
+        // chunk c of the solve's block s: op(A)[block, 16 k] and those k of X.  The solved rows
+        // are [0, kb) for a lower op(A), [kb + sz, n) for an upper one; the chunks run from the
+        // rows solved first, so that the first ones of the next block are ready early.
+        auto stage = [&](int s, int c) {
+            const int kb = (upper ? nblk - 1 - s : s) * kTB, sz = min(kTB, n - kb);
+            const int k1 = upper ? n : kb, kfirst = upper ? kb + sz : 0, nch = (k1 - kfirst + kLlK - 1) / kLlK;
+            double* As = ring + (c % kLlStages) * kLlStage;
+            double* Xs = As + kLlK * kLlPA;
+            const int kc = kfirst + (upper ? nch - 1 - c : c) * kLlK, kw = min(kLlK, k1 - kc);
+            // op(A)[kb + row][kc + k] -> As[k][row], four elements a thread at fixed strides
+            const int ar = trans == 'N' ? t % kTB : t / kLlK, ak = trans == 'N' ? t / kTB : t % kLlK;
+            const int dr = trans == 'N' ? 0 : kThreads / kLlK, dk = trans == 'N' ? kThreads / kTB : 0;
+            const double* src = A + (kb + ar) * rs + (kc + ak) * ks;
+            const long step = dr * rs + dk * ks;
+            uint32_t dst = smem_u32(As + ak * kLlPA + ar);
+            const uint32_t dstep = (dk * kLlPA + dr) * 8;
+            if (sz == kTB && kw == kLlK) {
+#pragma unroll
+                for (int u = 0; u < kTB * kLlK / kThreads; ++u) cp_async_8(dst + u * dstep, src + u * step, 8);
+            } else {
+#pragma unroll
+                for (int u = 0; u < kTB * kLlK / kThreads; ++u) {
+                    const bool in = ar + u * dr < sz && ak + u * dk < kw;
+                    cp_async_8(dst + u * dstep, in ? src + u * step : A, in ? 8 : 0);
+                }
+            }
+            // X(kc + k, col) = B(kc + k, col) -> Xs[col][k]
+            const int xk = t % kLlK, xc = t / kLlK;
+            const double* xsrc = B + (kc + xk) + (long)xc * lb;
+            dst = smem_u32(Xs + xc * kLlPX + xk);
+#pragma unroll
+            for (int u = 0; u < kLlK * kTrsmCols / kThreads; ++u) {
+                const bool in = xk < kw && xc + u * (kThreads / kLlK) < r;
+                cp_async_8(dst + u * (kThreads / kLlK) * kLlPX * 8, in ? xsrc + u * (kThreads / kLlK) * lb : B, in ? 8 : 0);
+            }
+        };
+        int ahead = 0;  // chunks of this block already loading
         for (int s = 0; s < nblk; ++s) {
-            const int bi = upper ? nblk - 1 - s : s;
-            const int kb = bi * kTB, sz = min(kTB, n - kb);
-            // diagonal block: stored triangle of op(A), zero elsewhere (unit diagonal set below)
-            for (int e = t; e < kTB * kTB; e += kThreads) {
-                const int rr = e % kTB, cc = e / kTB;
-                const bool in = rr < sz && cc < sz && (upper ? rr <= cc : rr >= cc) && !(unit && rr == cc);
-                const int ar = trans == 'N' ? kb + rr : kb + cc, ac = trans == 'N' ? kb + cc : kb + rr;
-                cp_async_el(&D[rr][cc], A + ar + (long)ac * la, A, in);
+            const int kb = (upper ? nblk - 1 - s : s) * kTB, sz = min(kTB, n - kb);
+            const int nch = ((upper ? n - kb - sz : kb) + kLlK - 1) / kLlK;
+            // diagonal block in solve order, packed: element (sr, sc), sc <= sr, at base + sr dr + sc dc;
+            // a warp takes every eighth line along A's contiguous index (the diagonal of a unit
+            // triangle is not read)
+            {
+                const long dr = upper ? -rs : rs, dc = upper ? -ks : ks;
+                const double* base = A + (kb + (upper ? sz - 1 : 0)) * (rs + ks);
+                const long along = trans == 'N' ? dr : dc, across = trans == 'N' ? dc : dr;
+                const double* src = base + lane * along + warp * across;
+                for (int line = warp; line < sz; line += 8, src += 8 * across)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int i = lane + 32 * h, sr = trans == 'N' ? i : line, sc = trans == 'N' ? line : i;
+                        if (i < sz && (unit ? sc < sr : sc <= sr))
+                            cp_async_8(smem_u32(D + tri_at(sr, sc)), src + 32 * h * along, 8);
+                    }
+                if (sz < kTB)  // solve rows past the block: zeros
+                    for (int e = t; e < kTB * kTB; e += kThreads) {
+                        const int sr = e / kTB, sc = e % kTB;
+                        if (sr >= sz && sc <= sr) D[tri_at(sr, sc)] = 0.0;
+                    }
             }
             cp_async_commit();
-            // this thread's B values of the block (DMMA accumulator layout), loaded ahead
-            double bv[4][4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int row = 16 * rt + g + 8 * (v >> 1), col = 8 * (ct0 + u) + 2 * tq + (v & 1);
-                    bv[u][v] = (row < sz && col < r) ? B[kb + row + (long)col * lb] : 0.0;
-                }
-            // solved rows: [0, kb) for a lower op(A), [kb + sz, n) for an upper one
-            const int k0 = upper ? kb + sz : 0, k1 = upper ? n : kb;
-            const int nch = (k1 - k0 + kLlK - 1) / kLlK;
-            auto stage = [&](int c) {
-                double(*As)[kLlPitch] = reinterpret_cast<double(*)[kLlPitch]>(ring + (c & 1) * kLlStage);
-                double(*Xs)[kLlPitch] = As + kLlK;
-                const int kc = k0 + c * kLlK, kw = min(kLlK, k1 - kc);
-                for (int e = t; e < kTB * kLlK; e += kThreads) {  // op(A)[kb + row][kc + k] -> As[k][row]
-                    int row, k;
-                    if (trans == 'N') row = e % kTB, k = e / kTB;
-                    else k = e % kLlK, row = e / kLlK;
-                    const int ar = trans == 'N' ? kb + row : kc + k, ac = trans == 'N' ? kc + k : kb + row;
-                    cp_async_el(&As[k][row], A + ar + (long)ac * la, A, row < sz && k < kw);
-                }
-                for (int e = t; e < kLlK * kMaxRhs; e += kThreads) {  // X[kc + k][col] = B(kc + k, col) -> Xs[k][col]
-                    const int k = e % kLlK, col = e / kLlK;
-                    cp_async_el(&Xs[k][col], B + (kc + k) + (long)col * lb, B, k < kw && col < r);
-                }
-            };
             double acc[4][4] = {};
-            if (nch > 0) stage(0);
-            cp_async_commit();
-            for (int c = 0; c < nch; ++c) {
-                if (c + 1 < nch) stage(c + 1);
+#pragma unroll
+            for (int c = 0; c < kLlStages - 1; ++c) {
+                if (c >= ahead && c < nch) stage(s, c);
                 cp_async_commit();
-                cp_async_wait<1>();
+            }
+            for (int c = 0; c < nch; ++c) {
+                cp_async_wait<kLlStages - 2>();
                 __syncthreads();
-                const double(*As)[kLlPitch] = reinterpret_cast<const double(*)[kLlPitch]>(ring + (c & 1) * kLlStage);
-                const double(*Xs)[kLlPitch] = As + kLlK;
-                if (ct0 < nct) {
+                if (c + kLlStages - 1 < nch) stage(s, c + kLlStages - 1);
+                cp_async_commit();
+                const double* As = ring + (c % kLlStages) * kLlStage;
+                const double* Xs = As + kLlK * kLlPA;
+                double af[4];
 #pragma unroll
-                    for (int k8 = 0; k8 < kLlK / 8; ++k8) {
-                        double af[4];
+                for (int v = 0; v < 4; ++v)
+                    af[v] = As[(8 * kh + tq + 4 * (v >> 1)) * kLlPA + 16 * rt + g + 8 * (v & 1)];
 #pragma unroll
-                        for (int v1 = 0; v1 < 2; ++v1)
+                for (int u = 0; u < 4; ++u) {
+                    if (u >= nct) break;
+                    double bf[2];
 #pragma unroll
-                            for (int v0 = 0; v0 < 2; ++v0) af[v0 + 2 * v1] = As[8 * k8 + tq + 4 * v1][16 * rt + g + 8 * v0];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            if (ct0 + u >= nct) break;
-                            double bf[2];
-#pragma unroll
-                            for (int v = 0; v < 2; ++v) bf[v] = Xs[8 * k8 + tq + 4 * v][8 * (ct0 + u) + g];
-                            dmma_16x8x8(acc[u], af, bf);
-                        }
-                    }
+                    for (int v = 0; v < 2; ++v) bf[v] = Xs[(8 * u + g) * kLlPX + 8 * kh + tq + 4 * v];
+                    dmma_16x8x8(acc[u], af, bf);
                 }
-                __syncthreads();
             }
             cp_async_wait<0>();
             __syncthreads();
-            // the block to solve: X = B_block - acc, zero outside sz x r
-            for (int e = t; e < kTB * kPP; e += kThreads) X[e / kPP][e % kPP] = 0.0;
-            if (unit && t < sz) D[t][t] = 1.0;
-            __syncthreads();
+            // the block to solve, in solve order: X = alpha B_block, then minus both halves' sums
+            if (t < kTB) dinv[t] = (unit || t >= sz) ? 1.0 : 1.0 / D[tri_at(t, t)];
+            {
+                double bv[kTB * kTrsmCols / kThreads];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const int row = 16 * rt + g + 8 * (v >> 1), col = 8 * (ct0 + u) + 2 * tq + (v & 1);
-                    if (ct0 + u < nct && row < sz && col < r) X[row][col] = bv[u][v] - acc[u][v];
+                for (int u = 0; u < kTB * kTrsmCols / kThreads; ++u) {
+                    const int e = u * kThreads + t, rr = e % kTB, cc = e / kTB;
+                    bv[u] = (rr < sz && cc < r) ? B[kb + (upper ? sz - 1 - rr : rr) + (long)cc * lb] : 0.0;
                 }
-            if (t < kTB) dinv[t] = (unit || t >= sz) ? 1.0 : 1.0 / D[t][t];
+#pragma unroll
+                for (int u = 0; u < kTB * kTrsmCols / kThreads; ++u) {
+                    const int e = u * kThreads + t;
+                    X[e % kTB][e / kTB] = alpha * bv[u];
+                }
+            }
             __syncthreads();
+            if (!unit)  // columns of D times 1 / diagonal
+                for (int e = t; e < kLlTri; e += kThreads) {
+                    const int row = e / (kTB + 1), j = e % (kTB + 1);
+                    D[e] *= dinv[j <= kTB - 1 - row ? j : kTB - j];
+                }
+            if (nch > 0)
+                for (int h = 0; h < 2; ++h) {
+                    if (kh == h) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u)
+#pragma unroll
+                            for (int v = 0; v < 4; ++v) {
+                                const int row = 16 * rt + g + 8 * (v >> 1), col = 8 * u + 2 * tq + (v & 1);
+                                if (u < nct && row < sz) X[upper ? sz - 1 - row : row][col] -= acc[u][v];
+                            }
+                    }
+                    __syncthreads();
+                }
+            else
+                __syncthreads();
+            // the next block's first kLlAhead chunks, if none of their rows is this block's: they
+            // are the first ones of a lower triangle's solved rows and the last ones of an upper's
+            const int solved = upper ? n - kb - sz : kb;  // rows before this block, in solve order
+            ahead = s + 1 < nblk && solved >= (kLlAhead + 1) * kLlK ? kLlAhead : 0;
+            for (int c = 0; c < ahead; ++c) stage(s + 1, c);
             // substitution: warp w holds right-hand sides w + 8 c for the c < cw it has
-            // (cw rounded up to 1, 2, 4 or 8 slots; a warp without columns skips it)
-            substitute_rhs<double>(X, D, dinv, sz, upper, r);
+            const int cw = r > warp ? (r - warp + 7) / 8 : 0;
+            if (cw > 2)
+                substitute_packed<4>(X, D, dinv, sz);
+            else if (cw > 1)
+                substitute_packed<2>(X, D, dinv, sz);
+            else if (cw == 1)
+                substitute_packed<1>(X, D, dinv, sz);
             __syncthreads();
             for (int e = t; e < kTB * r; e += kThreads) {
                 const int rr = e % kTB, cc = e / kTB;
-                if (rr < sz) B[kb + rr + (long)cc * lb] = X[rr][cc];
+                if (rr < sz) B[kb + (upper ? sz - 1 - rr : rr) + (long)cc * lb] = X[rr][cc];
             }
             __syncthreads();  // the solved rows are visible to the next block's copies
         }
@@ -837,12 +941,12 @@ cudaError_t launch_gemm_batched(const BatchDevice& d, int dtype, char transa, ch
     return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_trsm_batched(const int* order, int count, int* next, const int* dims, int dtype, char uplo,
+cudaError_t launch_trsm_batched(const int2* items, int count, int* next, const int* dims, int dtype, char uplo,
                                 char trans, char diag, const void* alpha, const void* const* a, const int* lda,
                                 void* const* b, const int* ldb, int grid, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
     const int sm = (3 * kTB * (kTB + 4) + kTB) * (dtype == BATCH_F64 ? 8 : 4);
-    const int sm_ll = (kLlRing + kTB * kTP + kTB) * 8;
+    const int sm_ll = (kLlRing + kLlTri + kTB) * 8;
     cudaError_t e = dtype == BATCH_F64 ? ensure_dynamic_smem(trsm_batched_ll_f64, sm_ll)
                                        : ensure_dynamic_smem(trsm_batched_kernel<float>, sm);
     if (e != cudaSuccess) return e;
@@ -850,11 +954,11 @@ cudaError_t launch_trsm_batched(const int* order, int count, int* next, const in
     prof_begin(st);
     if (dtype == BATCH_F64)
         trsm_batched_ll_f64<<<grid, kThreads, sm_ll, st>>>(
-            order, count, next, dims, uplo, trans, diag, *static_cast<const double*>(alpha),
+            items, count, next, dims, uplo, trans, diag, *static_cast<const double*>(alpha),
             reinterpret_cast<const double* const*>(a), lda, reinterpret_cast<double* const*>(b), ldb);
     else
         trsm_batched_kernel<float><<<grid, kThreads, sm, st>>>(
-            order, count, next, dims, uplo, trans, diag, *static_cast<const float*>(alpha),
+            items, count, next, dims, uplo, trans, diag, *static_cast<const float*>(alpha),
             reinterpret_cast<const float* const*>(a), lda, reinterpret_cast<float* const*>(b), ldb);
     count_launch();
     prof_end(st);

@@ -35,9 +35,13 @@ cudaError_t launch_gemm_batched(const BatchDevice& d, int dtype, char transa, ch
                                 const void* const* a, const int* lda, const void* const* b, const int* ldb,
                                 const void* beta, void* const* c, const int* ldc, int grid, cudaStream_t st);
 
-// order: problems longest first (CTAs claim them through the counter `next`, zeroed
-// by the launch); dims: n, nrhs per problem.
-cudaError_t launch_trsm_batched(const int* order, int count, int* next, const int* dims, int dtype, char uplo,
+// FP64 TRSM work items: right-hand sides of one item, and their CTAs per SM.
+constexpr int kTrsmCols = 32;
+constexpr int kTrsmCtasPerSm = 3;
+
+// items: (problem, first column), longest first (CTAs claim them through the counter `next`,
+// zeroed by the launch); FP32 items are whole problems; dims: n, nrhs per problem.
+cudaError_t launch_trsm_batched(const int2* items, int count, int* next, const int* dims, int dtype, char uplo,
                                 char trans, char diag, const void* alpha, const void* const* a, const int* lda,
                                 void* const* b, const int* ldb, int grid, cudaStream_t st);
 

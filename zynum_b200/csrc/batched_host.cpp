@@ -152,8 +152,9 @@ struct Batch {
     int* d_dims = nullptr;
     BatchWork* d_work = nullptr;  // GEMM work items, followed by the claim counter
     int* d_next = nullptr;        // claim counter (after the GEMM items or the TRSM order)
-    int* d_order = nullptr;
-    int n_items = 0;
+    int2* d_order = nullptr;      // TRSM work items
+    int n_items = 0;              // GEMM work items / non-empty TRSM problems
+    int n_launch = 0;             // TRSM work items
     int cfg_counts[3] = {0, 0, 0};
     // graph replay
     cudaGraphExec_t exec = nullptr;
@@ -448,33 +449,43 @@ int zynum_blas_gpu_trsm_batch_create(zynum_blas_gpu_batch_t* out, int dtype, cha
     b->count = count;
     b->m.assign(m, m + count);
     b->n.assign(n, n + count);
-    b->grid = 2 * sm_count();  // two solver CTAs per SM (registers and shared memory allow it)
+    // solver CTAs per SM: registers and shared memory allow three (FP64), two (FP32)
+    b->grid = (dtype == BATCH_F64 ? kTrsmCtasPerSm : 2) * sm_count();
     std::vector<int> dims;
-    std::vector<double> cost;
+    struct Item {
+        int2 at;
+        double cost;
+    };
+    std::vector<Item> items;  // empty problems left out
     for (int q = 0; q < count; ++q) {
         dims.push_back(m[q]);
         dims.push_back(n[q]);
-        // modelled solver time (us): per 64-row block a substitution and set-up (~5 us),
-        // per chunk update a fixed part (panel wait, loads, barriers ~2 us) plus the
-        // products (~4.2 us for 64 right-hand sides)
-        const double nb = (m[q] + 63) / 64;
-        cost.push_back(nb * (nb - 1.0) / 2.0 * (2.0 + 0.066 * n[q]) + 5.0 * nb + 1.0);
+        if (m[q] <= 0 || n[q] <= 0) continue;
+        ++b->n_items;
+        const int step = dtype == BATCH_F64 ? kTrsmCols : n[q];
+        for (int c0 = 0; c0 < n[q]; c0 += step) {
+            // modelled solver time (us): per 64-row block a substitution and set-up (~5 us),
+            // per chunk update a fixed part (panel wait, loads, barriers ~2 us) plus the
+            // products (~4.2 us for 64 right-hand sides)
+            const double nb = (m[q] + 63) / 64;
+            items.push_back({make_int2(q, c0),
+                             nb * (nb - 1.0) / 2.0 * (2.0 + 0.066 * std::min(step, n[q] - c0)) + 5.0 * nb + 1.0});
+        }
     }
-    // longest first (empty problems left out): the kernel's CTAs claim problems in this order
-    std::vector<int> order;
-    for (int q = 0; q < count; ++q)
-        if (m[q] > 0 && n[q] > 0) order.push_back(q);
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-    b->n_items = (int)order.size();
+    // longest first: the kernel's CTAs claim items in this order
+    std::stable_sort(items.begin(), items.end(), [](const Item& x, const Item& y) { return x.cost > y.cost; });
+    std::vector<int2> order;
+    for (const Item& it : items) order.push_back(it.at);
+    b->n_launch = (int)order.size();
     cudaError_t e = cudaSuccess;
     if (count) {
         if ((e = cudaMalloc(&b->d_dims, dims.size() * sizeof(int))) == cudaSuccess)
             e = cudaMemcpy(b->d_dims, dims.data(), dims.size() * sizeof(int), cudaMemcpyHostToDevice);
         // the order, then the claim counter (16-byte aligned after it)
-        const size_t order_bytes = (order.size() * sizeof(int) + 15) / 16 * 16;
+        const size_t order_bytes = (order.size() * sizeof(int2) + 15) / 16 * 16;
         if (e == cudaSuccess && (e = cudaMalloc(&b->d_order, order_bytes + 16)) == cudaSuccess) {
-            b->d_next = b->d_order + order_bytes / sizeof(int);
-            e = cudaMemcpy(b->d_order, order.data(), order.size() * sizeof(int), cudaMemcpyHostToDevice);
+            b->d_next = reinterpret_cast<int*>(reinterpret_cast<char*>(b->d_order) + order_bytes);
+            e = cudaMemcpy(b->d_order, order.data(), order.size() * sizeof(int2), cudaMemcpyHostToDevice);
         }
     }
     if (e != cudaSuccess) {
@@ -543,7 +554,7 @@ ZB_GEMM_BATCH_RUN(zynum_blas_gpu_sgemm_batch_run, float, BATCH_F32)
         args.b = b;                                                                                                 \
         args.ldb = ldb;                                                                                             \
         auto fn = [&](cudaStream_t s) {                                                                             \
-            return launch_trsm_batched(bt->d_order, bt->n_items, bt->d_next, bt->d_dims, DT, bt->uplo, bt->ta,     \
+            return launch_trsm_batched(bt->d_order, bt->n_launch, bt->d_next, bt->d_dims, DT, bt->uplo, bt->ta,     \
                                        bt->diag, &alpha, (const void* const*)a, lda, (void* const*)b, ldb, bt->grid, \
                                        s);                                                                           \
         };                                                                                                          \
