@@ -66,22 +66,35 @@ ZB_DEVICE T op_tri(const T* a, long lda, char uplo, char trans, char diag, int r
 }
 
 // Block b: inverse of the diagonal block op(A)[b*64 .. , b*64 ..] of size
-// s <= 64, written column-major with ld 64 (zero outside s x s).  Column j of
-// the inverse is solved by the four lanes of quad j % 8 of warp j / 8 (256
-// threads): for each row in solve order the lanes add every fourth term of
+// s <= 64, written column-major with ld 64 (zero outside s x s).  An upper block
+// is turned around (row and column i become 63 - i), so that every inverse is a
+// lower one.  The four 16 x 16 diagonal blocks by substitution, column j by the
+// four lanes of a quad: for each row the lanes add every fourth term of
 // sum_q L[r][q] X[q][j], two shuffles combine them, and the row's reciprocal
-// diagonal (computed once per block) scales the result.
+// diagonal (computed once) scales the result.  Then two levels of
+// X21 = -X22 (L21 X11), 16 and 32 wide.  Bound: latency (64 serial steps of
+// substitution took 32 us for order 4096, cold; sixteen and the merges 13.6).
+constexpr int kTriT = 32;  // scratch of a merge: 32 x 33
+
+template <typename T>
+__host__ __device__ constexpr int tri_inv_smem() {
+    return (2 * kNB * (kNB + 1) + kTriT * (kTriT + 1) + kNB) * (int)sizeof(T);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) tri_inv_blocks(const T* __restrict__ a, long lda, char uplo, char trans,
                                                       char diag, int n, T* __restrict__ out) {
-    extern __shared__ __align__(16) unsigned char tri_smem[];  // 2 x 64 x 65 elements + 64 reciprocals
+    extern __shared__ __align__(16) unsigned char tri_smem[];  // 2 x 64 x 65 elements, a merge's scratch, 64 reciprocals
     T(*L)[kNB + 1] = reinterpret_cast<T(*)[kNB + 1]>(tri_smem);
     T(*X)[kNB + 1] = L + kNB;
-    T* dinv = reinterpret_cast<T*>(X + kNB);
+    T(*W)[kTriT + 1] = reinterpret_cast<T(*)[kTriT + 1]>(X + kNB);
+    T* dinv = reinterpret_cast<T*>(W + kTriT);
     grid_dependency_wait();  // may start during the tail of the kernel before it (which may write A)
     const int b0 = blockIdx.x * kNB;
     const int s = min(kNB, n - b0);
     const int t = threadIdx.x;
+    const bool upper = op_is_upper(uplo, trans);
+    auto turned = [&](int i) { return upper ? kNB - 1 - i : i; };
     // all sixteen loads of a thread in flight before the first shared store
     constexpr int kIt = kNB * kNB / 256;
     T pre[kIt];
@@ -92,34 +105,55 @@ __global__ void __launch_bounds__(256) tri_inv_blocks(const T* __restrict__ a, l
     }
 #pragma unroll
     for (int i = 0; i < kIt; ++i) {
-        const int q = i * 256 + t, r = q % kNB, c = q / kNB;
+        const int q = i * 256 + t, r = turned(q % kNB), c = turned(q / kNB);
         L[r][c] = pre[i];
         X[r][c] = T(0);
     }
     __syncthreads();
-    if (t < kNB) dinv[t] = (t < s && diag != 'U') ? T(1) / L[t][t] : T(1);
+    if (t < kNB) dinv[t] = (turned(t) < s && diag != 'U') ? T(1) / L[t][t] : T(1);
     __syncthreads();
-    const bool upper = op_is_upper(uplo, trans);
-    const int lane = t & 31, j = (t >> 5) * 8 + (lane >> 2), part = lane & 3;
-    for (int step = 0; step < kNB; ++step) {
-        const int r = upper ? kNB - 1 - step : step;
-        const bool active = j < s && r < s && (upper ? r <= j : r >= j);
-        T v = T(0);
-        if (active) {
-            if (!upper) {
+    {
+        const int lane = t & 31, j = (t >> 5) * 8 + (lane >> 2), part = lane & 3, first = j & ~15;
+        for (int r = first; r < first + 16; ++r) {
+            T v = T(0);
+            if (r >= j)
                 for (int q = j + part; q < r; q += 4) v = fma(L[r][q], X[q][j], v);
-            } else {
-                for (int q = r + 1 + part; q <= j; q += 4) v = fma(L[r][q], X[q][j], v);
-            }
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (r >= j && part == 0) X[r][j] = ((r == j ? T(1) : T(0)) - v) * dinv[r];
+            __syncwarp();
         }
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        v += __shfl_xor_sync(0xffffffffu, v, 2);
-        if (active && part == 0) X[r][j] = ((r == j ? T(1) : T(0)) - v) * dinv[r];
-        __syncwarp();
     }
     __syncthreads();
+    // X21 = -X22 (L21 X11) for blocks of h rows; each thread one row, `w` columns of one product
+    auto merge = [&](int h, int o, int i, int j0, int w, int wrow) {
+        T v[4];
+        for (int u = 0; u < w; ++u) v[u] = T(0);
+        for (int q = j0; q < h; ++q) {  // X11 is lower: an Inf or NaN of L21 meets no zero of it
+            const T l = L[o + h + i][o + q];
+            for (int u = 0; u < w; ++u)
+                if (q >= j0 + u) v[u] = fma(l, X[o + q][o + j0 + u], v[u]);
+        }
+        for (int u = 0; u < w; ++u) W[wrow + i][j0 + u] = v[u];
+        __syncthreads();
+        for (int u = 0; u < w; ++u) v[u] = T(0);
+        for (int q = 0; q <= i; ++q) {
+            const T l = X[o + h + i][o + h + q];
+            for (int u = 0; u < w; ++u) v[u] = fma(l, W[wrow + q][j0 + u], v[u]);
+        }
+        for (int u = 0; u < w; ++u) X[o + h + i][o + j0 + u] = T(0) - v[u];
+        __syncthreads();
+    };
+    {
+        const int pair = t >> 7, tt = t & 127;  // two pairs of 16 x 16 blocks, two columns a thread
+        merge(16, 32 * pair, tt >> 3, 2 * (tt & 7), 2, 16 * pair);
+        merge(32, 0, t >> 3, 4 * (t & 7), 4, 0);
+    }
     T* o = out + (long)blockIdx.x * kNB * kNB;
-    for (int q = t; q < kNB * kNB; q += 256) o[q] = X[q % kNB][q / kNB];
+    for (int q = t; q < kNB * kNB; q += 256) {
+        const int r = q % kNB, c = q / kNB;
+        o[q] = (r < s && c < s) ? X[turned(r)][turned(c)] : T(0);
+    }
 }
 
 // One TRSM leaf of up to kLeaf rows (up to four diagonal 64-blocks), solved in
@@ -250,11 +284,13 @@ ZB_DEVICE double staged(const double (*W)[kStagePitch], bool rfast, int r, int c
     return rfast ? W[c][r] : W[r][c];
 }
 
-// acc[u] += A (64 x 64, staged) * B (64 x 64 in X[k][c]) for this warp's tiles:
-// row tile rt = warp / 2, column tiles 4 (warp % 2) + u.
-ZB_DEVICE void mma_64(double (&acc)[4][4], const double (*A)[kStagePitch], bool arfast, const double (*B)[kNB + 1]) {
+// acc[u] += A (64 x 64, staged) * B (64 x kInvCols in X[k][c]) for this warp's tiles:
+// row tile rt = warp / 2, column tiles 2 (warp % 2) + u.
+constexpr int kInvCols = 32;
+ZB_DEVICE void mma_64(double (&acc)[2][4], const double (*A)[kStagePitch], bool arfast,
+                      const double (*B)[kInvCols + 1]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, tq = lane & 3, rt = warp >> 1, ct0 = (warp & 1) * 4;
+    const int g = lane >> 2, tq = lane & 3, rt = warp >> 1, ct0 = (warp & 1) * 2;
 #pragma unroll
     for (int kb = 0; kb < kNB / 8; ++kb) {
         double af[4];
@@ -264,7 +300,7 @@ ZB_DEVICE void mma_64(double (&acc)[4][4], const double (*A)[kStagePitch], bool 
             for (int v0 = 0; v0 < 2; ++v0)
                 af[v0 + 2 * v1] = staged(A, arfast, 16 * rt + g + 8 * v0, 8 * kb + tq + 4 * v1);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 2; ++u) {
             double bf[2];
 #pragma unroll
             for (int v = 0; v < 2; ++v) bf[v] = B[8 * kb + tq + 4 * v][8 * (ct0 + u) + g];
@@ -273,25 +309,26 @@ ZB_DEVICE void mma_64(double (&acc)[4][4], const double (*A)[kStagePitch], bool 
     }
 }
 
-// Block (leaf, j): column block j of the inverse of the diagonal kLeaf-block
-// `leaf` of op(A), written to inv_leaf + leaf kLeaf^2 (column-major, ld kLeaf;
+// Block (leaf, j, h): kInvCols columns (half h) of column block j of the inverse of the
+// diagonal kLeaf-block `leaf` of op(A), written to inv_leaf + leaf kLeaf^2 (column-major, ld kLeaf;
 // zero outside the triangle and the leaf).  Lower op(A): X_jj = inv(A_jj),
 // X_ij = -inv(A_ii) sum_{k=j}^{i-1} A_ik X_kj for i = j+1, ...; upper op(A):
 // the same for i = j-1, ..., 0 with k = i+1 .. j.  The 64-blocks this takes
 // (inv(A_jj), then per row block i its A_ik and inv(A_ii)) are known up front:
 // they are staged through two shared buffers, the next one loading while the
 // current one is used (a load-then-use sequence waited out one L2 or DRAM
-// round trip per block).
+// round trip per block).  Column halves in their own CTAs: 128 CTAs for order 4096, each
+// with half of the up to nine dependent products (41 -> 27 us, cold).
 __global__ void __launch_bounds__(256)
 tri_inv_leaf(const double* __restrict__ a, long lda, int trans_n, int upper, int na, const double* __restrict__ inv64,
              double* __restrict__ inv_leaf) {
     extern __shared__ __align__(16) unsigned char til_smem[];
-    double(*X)[kNB][kNB + 1] = reinterpret_cast<double(*)[kNB][kNB + 1]>(til_smem);
+    double(*X)[kNB][kInvCols + 1] = reinterpret_cast<double(*)[kNB][kInvCols + 1]>(til_smem);
     double(*S0)[kStagePitch] =
-        reinterpret_cast<double(*)[kStagePitch]>(til_smem + sizeof(double) * 4 * kNB * (kNB + 1));
+        reinterpret_cast<double(*)[kStagePitch]>(til_smem + sizeof(double) * 4 * kNB * (kInvCols + 1));
     double(*S1)[kStagePitch] = S0 + kNB;
     grid_dependency_wait();  // launched during the tail of tri_inv_blocks
-    const int leaf = blockIdx.x, j = blockIdx.y, t = threadIdx.x;
+    const int leaf = blockIdx.x, j = blockIdx.y, h0 = blockIdx.z * kInvCols, t = threadIdx.x;
     const int P = leaf * kLeaf, len = min(kLeaf, na - P), nsb = (len + kNB - 1) / kNB;
     double* out = inv_leaf + (long)leaf * kLeaf * kLeaf;
     bool have[4] = {false, false, false, false};
@@ -331,8 +368,8 @@ tri_inv_leaf(const double* __restrict__ a, long lda, int trans_n, int upper, int
                 stage_block(Sb, ablock(i, k), sr, sc, len - i * kNB, len - k * kNB, a);
             cp_async_commit();
         };
-        const int lane = t & 31, warp = t >> 5, g = lane >> 2, tq = lane & 3, rt = warp >> 1, ct0 = (warp & 1) * 4;
-        double acc[4][4] = {};
+        const int lane = t & 31, warp = t >> 5, g = lane >> 2, tq = lane & 3, rt = warp >> 1, ct0 = (warp & 1) * 2;
+        double acc[2][4] = {};
         issue(0);
         for (int s = 0; s < nsteps; ++s) {
             if (s + 1 < nsteps) {
@@ -347,30 +384,31 @@ tri_inv_leaf(const double* __restrict__ a, long lda, int trans_n, int upper, int
             int i, k;
             info(s, inv_step, i, k);
             if (s == 0) {  // X_jj = inv(A_jj)
-                for (int q = t; q < kNB * kNB; q += 256) X[j][q % kNB][q / kNB] = staged(Sb, true, q % kNB, q / kNB);
+                for (int q = t; q < kNB * kInvCols; q += 256)
+                    X[j][q % kNB][q / kNB] = staged(Sb, true, q % kNB, h0 + q / kNB);
                 have[j] = true;
             } else if (!inv_step) {  // acc += A_ik X_kj; after the last k the sum goes to X[i]
                 const int k0 = upper ? i + 1 : j, k1 = upper ? j : i - 1;
                 if (k == k0) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < 2; ++u)
 #pragma unroll
                         for (int v = 0; v < 4; ++v) acc[u][v] = 0.0;
                 }
                 mma_64(acc, Sb, sr == 1, X[k]);
                 if (k == k1) {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u)
+                    for (int u = 0; u < 2; ++u)
 #pragma unroll
                         for (int v = 0; v < 4; ++v)
                             X[i][16 * rt + g + 8 * (v >> 1)][8 * (ct0 + u) + 2 * tq + (v & 1)] = acc[u][v];
                 }
             } else {  // X_ij = -inv(A_ii) * sum
-                double y[4][4] = {};
+                double y[2][4] = {};
                 mma_64(y, Sb, true, X[i]);
                 __syncthreads();
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
+                for (int u = 0; u < 2; ++u)
 #pragma unroll
                     for (int v = 0; v < 4; ++v)
                         X[i][16 * rt + g + 8 * (v >> 1)][8 * (ct0 + u) + 2 * tq + (v & 1)] = -y[u][v];
@@ -380,9 +418,9 @@ tri_inv_leaf(const double* __restrict__ a, long lda, int trans_n, int upper, int
         }
     }
     // column block j of the leaf inverse: rows of computed blocks, zeros elsewhere
-    for (int q = t; q < kLeaf * kNB; q += 256) {
+    for (int q = t; q < kLeaf * kInvCols; q += 256) {
         const int r = q % kLeaf, c = q / kLeaf, bi = r / kNB;
-        out[r + (long)(j * kNB + c) * kLeaf] = (j < nsb && have[bi]) ? X[bi][r % kNB][c] : 0.0;
+        out[r + (long)(j * kNB + h0 + c) * kLeaf] = (j < nsb && have[bi]) ? X[bi][r % kNB][c] : 0.0;
     }
 }
 
@@ -782,7 +820,7 @@ cudaError_t trsm(const TrsmArgs<T>& t, void* planes, const GemmFn<T>& gemm, cuda
     const bool have_given = given != nullptr && std::is_same<T, double>::value;
     const bool given_t = have_given && given->transposed;
     if (!have_given) {
-        const int tri_smem = (2 * kNB * (kNB + 1) + kNB) * (int)sizeof(T);
+        const int tri_smem = tri_inv_smem<T>();
         if ((e = ensure_dynamic_smem(tri_inv_blocks<T>, tri_smem)) != cudaSuccess) return e;
         if ((e = launch_dependent(tri_inv_blocks<T>, dim3(nblk), dim3(256), (size_t)tri_smem, st, t.a, t.lda, t.uplo,
                                   t.trans, t.diag, na, inv)) != cudaSuccess)
@@ -822,9 +860,9 @@ cudaError_t trsm(const TrsmArgs<T>& t, void* planes, const GemmFn<T>& gemm, cuda
         const int nleaf = (na + kLeaf - 1) / kLeaf;
         double* built = reinterpret_cast<double*>(static_cast<char*>(planes) + inv_plane_bytes<T>(na));
         inv_leaf = built;
-        const int til_smem = (int)sizeof(double) * (4 * kNB * (kNB + 1) + 2 * kNB * kStagePitch);
+        const int til_smem = (int)sizeof(double) * (4 * kNB * (kInvCols + 1) + 2 * kNB * kStagePitch);
         if ((e = ensure_dynamic_smem(tri_inv_leaf, til_smem)) != cudaSuccess) return e;
-        if ((e = launch_dependent(tri_inv_leaf, dim3(nleaf, kLeaf / kNB), dim3(256), (size_t)til_smem, st,
+        if ((e = launch_dependent(tri_inv_leaf, dim3(nleaf, kLeaf / kNB, kNB / kInvCols), dim3(256), (size_t)til_smem, st,
                                   reinterpret_cast<const double*>(t.a), lda, (int)(ta == 'N'), (int)upper, na,
                                   reinterpret_cast<const double*>(inv), built)) != cudaSuccess)
             return e;
@@ -924,15 +962,15 @@ cudaError_t trsm_leaf_inverses(char uplo, char diag, int n, const double* a, lon
     cudaError_t e;
     double* inv = static_cast<double*>(scratch);
     const int nblk = (n + kNB - 1) / kNB, nleaf = (n + kLeaf - 1) / kLeaf;
-    const int tri_smem = (2 * kNB * (kNB + 1) + kNB) * (int)sizeof(double);
+    const int tri_smem = tri_inv_smem<double>();
     if ((e = ensure_dynamic_smem(tri_inv_blocks<double>, tri_smem)) != cudaSuccess) return e;
     if ((e = launch_dependent(tri_inv_blocks<double>, dim3(nblk), dim3(256), (size_t)tri_smem, st, a, lda, uplo, 'N',
                               diag, n, inv)) != cudaSuccess)
         return e;
     count_launch();
-    const int til_smem = (int)sizeof(double) * (4 * kNB * (kNB + 1) + 2 * kNB * kStagePitch);
+    const int til_smem = (int)sizeof(double) * (4 * kNB * (kInvCols + 1) + 2 * kNB * kStagePitch);
     if ((e = ensure_dynamic_smem(tri_inv_leaf, til_smem)) != cudaSuccess) return e;
-    if ((e = launch_dependent(tri_inv_leaf, dim3(nleaf, kLeaf / kNB), dim3(256), (size_t)til_smem, st, a, lda, 1,
+    if ((e = launch_dependent(tri_inv_leaf, dim3(nleaf, kLeaf / kNB, kNB / kInvCols), dim3(256), (size_t)til_smem, st, a, lda, 1,
                               (int)(uplo == 'U'), n, (const double*)inv, leaf)) != cudaSuccess)
         return e;
     count_launch();
