@@ -432,12 +432,19 @@ tri_inv_leaf(const double* __restrict__ a, long lda, int trans_n, int upper, int
 // rows are read by all four) and the cluster barrier orders those reads
 // before any CTA writes its rows back.  Warp w: row tile w / 2, column tile
 // w % 2, two accumulators.
+// Shared pitches: rows of the inverse 4 mod 16 doubles and Z 2 mod 16, so that fragment
+// loads are free of bank conflicts (2-way for Z, whose stores are along its other index):
+// TRSM 4096 x 512 572 -> 535 us against pitches of 2 and 1 mod 16, which made the loads
+// of a leaf cost twice its products.
+constexpr int kApZ = kLeafCols + 2, kApP = kNB + 4, kApT = kLeaf + 4;
+constexpr int kApSmem = (int)sizeof(double) * (kLeaf * kApZ + (kLeaf * kApP > kNB * kApT ? kLeaf * kApP : kNB * kApT));
+
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(256)
 trsm_leaf_apply(const double* __restrict__ inv_leaf, int left, int inv_t, int fwd, int p0, int len,
                 double* __restrict__ b, long ldb, int ncols, int wait_first) {
     extern __shared__ __align__(16) unsigned char ap_smem[];
-    double(*Z)[kLeafCols + 1] = reinterpret_cast<double(*)[kLeafCols + 1]>(ap_smem);
-    double* A = reinterpret_cast<double*>(ap_smem + sizeof(double) * kLeaf * (kLeafCols + 1));
+    double(*Z)[kApZ] = reinterpret_cast<double(*)[kApZ]>(ap_smem);
+    double* A = reinterpret_cast<double*>(ap_smem + sizeof(double) * kLeaf * kApZ);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = lane >> 2, tq = lane & 3;
     const int rb = (int)cluster_ctarank();
     const int c0 = (blockIdx.x / 4) * kLeafCols, nc = min(kLeafCols, ncols - c0);
@@ -446,22 +453,22 @@ trsm_leaf_apply(const double* __restrict__ inv_leaf, int left, int inv_t, int fw
     const int klen = max(0, kend - kbeg);
     const int klen8 = (klen + 7) & ~7;
     // rows 64 rb + i, columns kbeg + kk of inv(M): stored as is (inv_t = 0) inv[i' + k' kLeaf] (runs
-    // along i, staged [kk][i], pitch 66); stored transposed (inv_t = 1: side R, or an inverse of A
-    // serving op(A) = A^T) inv[k' + i' kLeaf] (runs along kk, staged [i][kk], pitch kLeaf + 2)
+    // along i, staged [kk][i]); stored transposed (inv_t = 1: side R, or an inverse of A
+    // serving op(A) = A^T) inv[k' + i' kLeaf] (runs along kk, staged [i][kk])
     if (wait_first) grid_dependency_wait();  // the kernel before this one wrote the inverses
     if (64 * rb < len && klen > 0) {
         if (!inv_t) {
             for (int q = t; q < klen8 * (kNB / 2); q += 256) {
                 const int kk = q / (kNB / 2), i = (q % (kNB / 2)) * 2;
                 const bool ok = kk < klen;
-                cp_async_16(smem_u32(A + kk * kStagePitch + i),
+                cp_async_16(smem_u32(A + kk * kApP + i),
                             ok ? inv_leaf + (kNB * rb + i) + (long)(kbeg + kk) * kLeaf : inv_leaf, ok ? 16 : 0);
             }
         } else {
             for (int q = t; q < kNB * (klen8 / 2); q += 256) {
                 const int i = q / (klen8 / 2), kk = (q % (klen8 / 2)) * 2;
                 const bool ok = kk < klen;
-                cp_async_16(smem_u32(A + i * (kLeaf + 2) + kk),
+                cp_async_16(smem_u32(A + i * kApT + kk),
                             ok ? inv_leaf + (kbeg + kk) + (long)(kNB * rb + i) * kLeaf : inv_leaf, ok ? 16 : 0);
             }
         }
@@ -501,7 +508,7 @@ trsm_leaf_apply(const double* __restrict__ inv_leaf, int left, int inv_t, int fw
 #pragma unroll
             for (int v0 = 0; v0 < 2; ++v0) {
                 const int i = 16 * rt + g + 8 * v0, kk = 8 * kb + tq + 4 * v1;
-                af[v0 + 2 * v1] = !inv_t ? A[kk * kStagePitch + i] : A[i * (kLeaf + 2) + kk];
+                af[v0 + 2 * v1] = !inv_t ? A[kk * kApP + i] : A[i * kApT + kk];
             }
 #pragma unroll
         for (int v = 0; v < 2; ++v) bf[v] = Z[kbeg + 8 * kb + tq + 4 * v][8 * ct + g];
@@ -853,8 +860,7 @@ cudaError_t trsm(const TrsmArgs<T>& t, void* planes, const GemmFn<T>& gemm, cuda
     const double* inv_leaf = nullptr;
     if (inv_leaves && have_given) {
         inv_leaf = given->leaf;
-        constexpr int kRows = kLeaf * kStagePitch > kNB * (kLeaf + 2) ? kLeaf * kStagePitch : kNB * (kLeaf + 2);
-        leaf_smem = (int)sizeof(double) * (kLeaf * (kLeafCols + 1) + kRows);
+        leaf_smem = kApSmem;
         e = ensure_dynamic_smem(trsm_leaf_apply, leaf_smem);
     } else if (inv_leaves) {
         const int nleaf = (na + kLeaf - 1) / kLeaf;
@@ -869,8 +875,7 @@ cudaError_t trsm(const TrsmArgs<T>& t, void* planes, const GemmFn<T>& gemm, cuda
         count_launch();
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         // Z plus 64 rows of the inverse over up to kLeaf columns (either staging layout)
-        constexpr int kRows = kLeaf * kStagePitch > kNB * (kLeaf + 2) ? kLeaf * kStagePitch : kNB * (kLeaf + 2);
-        leaf_smem = (int)sizeof(double) * (kLeaf * (kLeafCols + 1) + kRows);
+        leaf_smem = kApSmem;
         e = ensure_dynamic_smem(trsm_leaf_apply, leaf_smem);
     } else {
         leaf_smem = (int)sizeof(T) * (kLeaf * (kLeafCols + 1) + kNB * (kNB + 1));
