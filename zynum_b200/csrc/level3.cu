@@ -257,7 +257,7 @@ trsm_leaf(const T* __restrict__ a, long lda, int trans_n, int conj_a, int left, 
 // (one launch for all leaves, off the solve's critical chain); each leaf of
 // the solve is then one trsm_leaf_apply launch, Y = inv(M) Z, a single pass
 // of DMMA tiles with no dependent phases.
-constexpr int kStagePitch = kNB + 2;  // 66 doubles: 16-byte aligned shared rows
+constexpr int kStagePitch = kNB + 4;  // 16-byte aligned shared rows, fragment loads without bank conflicts
 
 // Stage the 64 x 64 block whose element (r, c) sits at base[r * sr + c * sc],
 // exactly one of sr / sc being 1, into W with the contiguous index innermost
@@ -286,9 +286,9 @@ ZB_DEVICE double staged(const double (*W)[kStagePitch], bool rfast, int r, int c
 
 // acc[u] += A (64 x 64, staged) * B (64 x kInvCols in X[k][c]) for this warp's tiles:
 // row tile rt = warp / 2, column tiles 2 (warp % 2) + u.
-constexpr int kInvCols = 32;
+constexpr int kInvCols = 32, kInvPitch = kInvCols + 4;
 ZB_DEVICE void mma_64(double (&acc)[2][4], const double (*A)[kStagePitch], bool arfast,
-                      const double (*B)[kInvCols + 1]) {
+                      const double (*B)[kInvPitch]) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, tq = lane & 3, rt = warp >> 1, ct0 = (warp & 1) * 2;
 #pragma unroll
@@ -323,9 +323,9 @@ __global__ void __launch_bounds__(256)
 tri_inv_leaf(const double* __restrict__ a, long lda, int trans_n, int upper, int na, const double* __restrict__ inv64,
              double* __restrict__ inv_leaf) {
     extern __shared__ __align__(16) unsigned char til_smem[];
-    double(*X)[kNB][kInvCols + 1] = reinterpret_cast<double(*)[kNB][kInvCols + 1]>(til_smem);
+    double(*X)[kNB][kInvPitch] = reinterpret_cast<double(*)[kNB][kInvPitch]>(til_smem);
     double(*S0)[kStagePitch] =
-        reinterpret_cast<double(*)[kStagePitch]>(til_smem + sizeof(double) * 4 * kNB * (kInvCols + 1));
+        reinterpret_cast<double(*)[kStagePitch]>(til_smem + sizeof(double) * 4 * kNB * kInvPitch);
     double(*S1)[kStagePitch] = S0 + kNB;
     grid_dependency_wait();  // launched during the tail of tri_inv_blocks
     const int leaf = blockIdx.x, j = blockIdx.y, h0 = blockIdx.z * kInvCols, t = threadIdx.x;
@@ -866,7 +866,7 @@ cudaError_t trsm(const TrsmArgs<T>& t, void* planes, const GemmFn<T>& gemm, cuda
         const int nleaf = (na + kLeaf - 1) / kLeaf;
         double* built = reinterpret_cast<double*>(static_cast<char*>(planes) + inv_plane_bytes<T>(na));
         inv_leaf = built;
-        const int til_smem = (int)sizeof(double) * (4 * kNB * (kInvCols + 1) + 2 * kNB * kStagePitch);
+        const int til_smem = (int)sizeof(double) * (4 * kNB * kInvPitch + 2 * kNB * kStagePitch);
         if ((e = ensure_dynamic_smem(tri_inv_leaf, til_smem)) != cudaSuccess) return e;
         if ((e = launch_dependent(tri_inv_leaf, dim3(nleaf, kLeaf / kNB, kNB / kInvCols), dim3(256), (size_t)til_smem, st,
                                   reinterpret_cast<const double*>(t.a), lda, (int)(ta == 'N'), (int)upper, na,
@@ -973,7 +973,7 @@ cudaError_t trsm_leaf_inverses(char uplo, char diag, int n, const double* a, lon
                               diag, n, inv)) != cudaSuccess)
         return e;
     count_launch();
-    const int til_smem = (int)sizeof(double) * (4 * kNB * (kInvCols + 1) + 2 * kNB * kStagePitch);
+    const int til_smem = (int)sizeof(double) * (4 * kNB * kInvPitch + 2 * kNB * kStagePitch);
     if ((e = ensure_dynamic_smem(tri_inv_leaf, til_smem)) != cudaSuccess) return e;
     if ((e = launch_dependent(tri_inv_leaf, dim3(nleaf, kLeaf / kNB, kNB / kInvCols), dim3(256), (size_t)til_smem, st, a, lda, 1,
                               (int)(uplo == 'U'), n, (const double*)inv, leaf)) != cudaSuccess)
