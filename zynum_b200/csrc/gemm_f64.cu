@@ -549,9 +549,10 @@ cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* wor
             if (use_tma_tiles(g, plan)) {
                 const int kc = dgemm_tma_k_chunk(g.k, splits);
                 const int used_t = (g.k + kc - 1) / kc;
-                if (used_t > 1 && !workspace) return cudaErrorInvalidValue;
-                cudaError_t e = dgemm_tma(g, splits, workspace, st);
-                if (e != cudaSuccess || used_t == 1) return e;
+                const bool cluster = used_t == 2 && plan.automatic;
+                if (used_t > 1 && !cluster && !workspace) return cudaErrorInvalidValue;
+                cudaError_t e = dgemm_tma(g, splits, workspace, cluster, st);
+                if (e != cudaSuccess || used_t == 1 || cluster) return e;
                 return splitk_reduce(g, used_t, workspace, st);
             }
             // op(B) k-contiguous (transb N): three 32-deep stages (212 KB), half the block

@@ -63,10 +63,11 @@ cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* wor
 // 16-byte aligned operands with even leading dimensions.  K is split into
 // ranges of dgemm_tma_k_chunk(k, splits) (a multiple of the 32-deep slice);
 // with more than one range the raw sums go to `workspace` (range z at
-// z * m * n, ld m) and the caller reduces them.
+// z * m * n, ld m) and the caller reduces them; with `cluster`, exactly two ranges are
+// summed between the two CTAs of a cluster and no workspace is used.
 bool dgemm_tma_applies(const GemmArgsF64& g);
 int dgemm_tma_k_chunk(int k, int splits);
-cudaError_t dgemm_tma(const GemmArgsF64& g, int splits, double* workspace, cudaStream_t st);
+cudaError_t dgemm_tma(const GemmArgsF64& g, int splits, double* workspace, bool cluster, cudaStream_t st);
 // Warp-specialised 64 x 64 DGEMM tiles (gemm_f64_ws.cu), K split over the CTAs of a
 // cluster of `splits` (1 or 2) that sum their partial tiles through distributed
 // shared memory: no workspace.  Needs dgemm_tma_applies(g).
