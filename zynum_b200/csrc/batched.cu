@@ -650,7 +650,7 @@ trsm_batched_kernel(const int2* __restrict__ items, int count, int* __restrict__
 // the split is for more independent blocks per SM and shorter chains: items of 32 columns
 // (a problem with 64 is two items and its chain half as long), the triangle packed into
 // 16.6 KB and a ring of 41 KB for three CTAs per SM.  5,000 problems (n 16..1024, 1..64
-// right-hand sides) 1.81 -> 1.45 ms, 1,800 of them 1.40 -> 0.98; with two 32-deep stages
+// right-hand sides) 1.81 -> 1.42 ms, 1,800 of them 1.40 -> 0.97; with two 32-deep stages
 // and whole problems on two CTAs before.  A fourth stage is slower (1.58 ms: it leaves L1 too
 // little), two stages or no chunk ahead 1.48 / 1.42 (the latter 3 % slower on small batches).
 constexpr int kLlK = 16;                               // K chunk
@@ -806,13 +806,44 @@ trsm_batched_ll_f64(const int2* __restrict__ items, int count, int* __restrict__
                 if (c >= ahead && c < nch) stage(s, c);
                 cp_async_commit();
             }
+            // From chunk kLlStages - 1 on, every chunk of a whole block has 16 k (an upper solve's
+            // ragged one is its first): its copies differ from the last chunk's by constants.
+            constexpr int kFirst = kLlStages - 1;
+            const int ar = trans == 'N' ? t % kTB : t / kLlK, ak = trans == 'N' ? t / kTB : t % kLlK;
+            const long astep = trans == 'N' ? (kThreads / kTB) * ks : (kThreads / kLlK) * rs;
+            const uint32_t adst = smem_u32(ring + ak * kLlPA + ar);
+            const uint32_t adstep = (trans == 'N' ? (kThreads / kTB) * kLlPA : kThreads / kLlK) * 8;
+            const int kc = upper ? kb + sz + (nch - 1 - kFirst) * kLlK : kFirst * kLlK;
+            const long anext = (upper ? -kLlK : kLlK) * ks;
+            const double* asrc = A + (kb + ar) * rs + (long)(kc + ak) * ks;
+            const int xc = t / kLlK;
+            const double* xsrc = B + (kc + t % kLlK) + (long)xc * lb;
+            const uint32_t xdst = smem_u32(ring + kLlK * kLlPA + xc * kLlPX + t % kLlK);
+            int slot = 0, fill = kFirst;  // of chunk c, of chunk c + kFirst
             for (int c = 0; c < nch; ++c) {
                 cp_async_wait<kLlStages - 2>();
                 __syncthreads();
-                if (c + kLlStages - 1 < nch) stage(s, c + kLlStages - 1);
+                if (c + kFirst < nch) {
+                    if (sz == kTB) {
+                        const uint32_t at = fill * (kLlStage * 8);
+#pragma unroll
+                        for (int u = 0; u < kTB * kLlK / kThreads; ++u)
+                            cp_async_8(adst + at + u * adstep, asrc + u * astep, 8);
+#pragma unroll
+                        for (int u = 0; u < kLlK * kTrsmCols / kThreads; ++u)
+                            if (xc + u * (kThreads / kLlK) < r)  // columns past r reach only outputs that are not used
+                                cp_async_8(xdst + at + u * (kThreads / kLlK) * kLlPX * 8, xsrc + u * (kThreads / kLlK) * lb, 8);
+                        asrc += anext;
+                        xsrc += upper ? -kLlK : kLlK;
+                    } else {
+                        stage(s, c + kFirst);
+                    }
+                }
                 cp_async_commit();
-                const double* As = ring + (c % kLlStages) * kLlStage;
+                const double* As = ring + slot * kLlStage;
                 const double* Xs = As + kLlK * kLlPA;
+                if (++slot == kLlStages) slot = 0;
+                if (++fill == kLlStages) fill = 0;
                 double af[4];
 #pragma unroll
                 for (int v = 0; v < 4; ++v)
@@ -857,7 +888,7 @@ trsm_batched_ll_f64(const int2* __restrict__ items, int count, int* __restrict__
 #pragma unroll
                             for (int v = 0; v < 4; ++v) {
                                 const int row = 16 * rt + g + 8 * (v >> 1), col = 8 * u + 2 * tq + (v & 1);
-                                if (u < nct && row < sz) X[upper ? sz - 1 - row : row][col] -= acc[u][v];
+                                if (u < nct && col < r && row < sz) X[upper ? sz - 1 - row : row][col] -= acc[u][v];
                             }
                     }
                     __syncthreads();
