@@ -478,14 +478,14 @@ static bool use_tma_tiles(const GemmArgsF64& g, const GemmPlan& plan) {
 // Cluster size with which a planned product runs on the 64 x 64 warp-specialised tiles
 // instead (dgemm_ws, which needs none of the plan's workspace); 0: it does not.
 static int ws_cluster(const GemmArgsF64& g, const GemmPlan& plan) {
-    if (!plan.automatic || !use_tma_operands(g)) return 0;
+    if (!plan.automatic) return 0;
     constexpr long sms = 148;
     const long t64 = (long)((g.m + 63) / 64) * ((g.n + 63) / 64);
     if (plan.tile == TILE_64x64) {
         // about one 64 x 64 tile per SM: two CTAs of a cluster per tile.  Fewer tiles keep the
         // cp.async tiles, which split K further and reduce through L2 (clusters of 4 and 8
         // lost to them: 384 x 384 x 1024 21.0 against 15.5 us, 256 x 256 x 1024 15.3 / 9.3).
-        return 4 * t64 > 2 * sms && 2 * t64 <= 2 * sms && g.k >= 256 ? 2 : 0;
+        return 4 * t64 > 2 * sms && 2 * t64 <= 2 * sms && g.k >= 256 && use_tma_operands(g) ? 2 : 0;
     }
     if (plan.tile != TILE_128x128 || plan.splits > 1 || g.k < 256) return 0;
     // both tile sizes run in rounds of one tile per SM; a 128 x 128 round at 0.955 of the
@@ -494,7 +494,7 @@ static int ws_cluster(const GemmArgsF64& g, const GemmPlan& plan) {
     const long m1 = (g.m + 127) / 128, n1 = (g.n + 127) / 128, m6 = (g.m + 63) / 64;
     const long live1 = g.tri ? m1 * (m1 + 1) / 2 : m1 * n1, live6 = g.tri ? m6 * (m6 + 1) / 2 : t64;
     const double r128 = 4.0 * ((live1 + sms - 1) / sms) / 0.955, r64 = ((live6 + sms - 1) / sms) / 0.90;
-    return r64 < 0.98 * r128 ? 1 : 0;
+    return r64 < 0.98 * r128 && use_tma_operands(g) ? 1 : 0;
 }
 
 // Cluster size with which a planned small product runs on the 64 x 64 cluster tiles

@@ -7,17 +7,20 @@
 // At k = n = 64 the product sits at the ridge of both pipes (2 k flop per
 // element of op(A)), so the math pipe has to keep working while HBM streams.
 // One persistent CTA of sixteen warps per SM stages op(B) once (zero-padded
-// to 64 x 64).  The warps form four independent groups of four, one warp of
-// each group per SM sub-partition; group g takes the CTA's row blocks g,
-// g + 4, ... and owns its own shared-memory stages, so the groups drift apart
-// and one group's loads and epilogue overlap the others' products.  There is
-// no producer warp: the group's first lane issues the group's TMA loads
-// (128-byte swizzle, zero fill past m and k) as soon as its four warps are
-// done with a stage, and the group's warps leave together through one
-// bar.red.and per block (bounded mbarrier waits; an abort drains the loads).
+// to 64 x 64).  The warps form independent groups (FP64 eight of two, FP32 four
+// of four); group g takes the CTA's row blocks g, g + groups, ... and owns its
+// own shared-memory stages, so the groups drift apart and one group's loads and
+// epilogue overlap the others' products.  There is no producer warp: the
+// group's first lane issues the group's TMA loads (128-byte swizzle, zero fill
+// past m and k) as soon as its warps are done with a stage, and the group's
+// warps leave together through one bar.red.and per block (bounded mbarrier
+// waits; an abort drains the loads).
 //
-// FP64: 32-row blocks, two stages per group (one block computed while the
-// next lands), DMMA m16n8k8 with each warp a 16 x 32 piece of the block;
+// FP64: 16-row blocks, two stages per group (one block computed while the
+// next lands), DMMA m16n8k8 with each warp a 16 x 32 piece of the block; eight
+// groups because a block's latencies (about five times its products) are only
+// hidden by other groups' products: four groups of four warps on 32-row blocks
+// took 55.3 / 45.5 us at 131072 x 64 x 64, beta 1 / 0, eight take 52.1 / 44.3;
 // fragment layouts and row / k / column bijections as in the 128 x 128 TMA
 // kernel (gemm_f64_tma.cu); beta * C is read into registers before the
 // block's products and C leaves by 16-byte streaming stores.  FP32: 128-row
@@ -25,7 +28,7 @@
 // fed by 16-byte shared loads.
 //
 // Measured at 131072 x 64 x 64 (timed in CUDA graphs) against cuBLAS on the
-// same layout: FP64 47.5 / 57.7 us (beta 0 / 1; cuBLAS 48.4 / 55.8), FP32
+// same layout: FP64 44.3 / 52.1 us (beta 0 / 1; cuBLAS 48.4 / 55.8), FP32
 // 35.1 / 36.5 us (cuBLAS 30.1 / 33.5).  Variants measured slower: a
 // dedicated producer warp with one or two groups of eight math warps (the
 // DMMA pipe idled while the lock-stepped warps ran their epilogues), TMA
@@ -47,23 +50,26 @@ namespace zb {
 namespace {
 
 constexpr int kKK = 64, kKN = 64;
-constexpr int kGroups = 4, kGroupWarps = 4, kGroupStages = 2;  // group g owns stages 2 g, 2 g + 1
+constexpr int kGroups = 8, kGroupWarps = 2, kGroupStages = 2;  // FP64; each group owns its stages
+constexpr int kFGroups = 4, kFGroupWarps = 4;                  // FP32, one stage each
 constexpr int kStagesAll = kGroups * kGroupStages;
 constexpr int kKThreads = kGroups * kGroupWarps * 32;
-constexpr int kKBM = 32;                                    // FP64 rows per block
-constexpr int kKABytes = kKBM * kKK * 8;                    // 16 KB per stage
+static_assert(kKThreads == kFGroups * kFGroupWarps * 32, "both kernels run the same block");
+constexpr int kKBM = 16;                                    // FP64 rows per block
+constexpr int kKABytes = kKBM * kKK * 8;                    // 8 KB per stage
 constexpr int kKBBytes = kKN * kKK * 8;                     // 32 KB, resident
 constexpr size_t kKSmem = 1024 + (size_t)kStagesAll * kKABytes + kKBBytes + 256;
 constexpr unsigned long long kKWaitNs = 4000000000ull;
 static_assert(kKK * kKN % kKThreads == 0, "op(B) staging: whole elements per thread");
 
-// Named barrier 1 + grp over the group's four warps; true iff every thread passed `ok`.
+// Named barrier 1 + grp over the group's warps; true iff every thread passed `ok`.
+template <int WARPS>
 ZB_DEVICE bool group_bar_and(int grp, bool ok) {
     uint32_t r;
     asm volatile(
         "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, %2, %3, p;\n selp.u32 %0, 1, 0, q;\n}\n"
         : "=r"(r)
-        : "r"((uint32_t)ok), "r"(1 + grp), "n"(kGroupWarps * 32)
+        : "r"((uint32_t)ok), "r"(1 + grp), "n"(WARPS * 32)
         : "memory");
     return r != 0;
 }
@@ -101,11 +107,11 @@ ZB_DEVICE uint32_t k_off(int mn, int k) {
     return (uint32_t)((k >> 4) * (R * 128) + mn * 128 + ((((k & 15) >> 1) ^ (mn & 7)) << 4) + ((k & 1) << 3));
 }
 
-// FP64: group g takes the CTA's row blocks g, g + 4, ... (32 rows each) and
+// FP64: group g takes the CTA's row blocks g, g + 8, ... (16 rows each) and
 // holds two of them in flight, one being computed while the next one's TMA
-// load lands.  Its four warps each own 16 rows x 32 columns of the block
-// (2 x 2 warps): four independent 16 x 8 DMMA accumulators per warp, and
-// sixteen per sub-partition with the four groups.
+// load lands.  Its two warps each own 16 rows x 32 columns of the block: four
+// independent 16 x 8 DMMA accumulators per warp, and sixteen per sub-partition
+// with the eight groups.
 template <bool A_MN, bool USE_C>
 __global__ void __launch_bounds__(kKThreads, 1)
 dgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ SkinnyParams P) {
@@ -163,7 +169,7 @@ dgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
     __syncthreads();
 
-    const int wm = (wq >> 1) * 16, wn = (wq & 1) * 32;
+    const int wm = 0, wn = wq * 32;
     const int g = lane >> 2, t = lane & 3;
     const int ks8 = (P.K + 7) / 8;
     const int nfrag = max(0, min(4, (P.N - wn + 7) / 8));  // 8-column fragments inside op(B)
@@ -235,7 +241,7 @@ dgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             }
         }
         // the group's four warps are done with the stage (or leave together)
-        if (!(ok = group_bar_and(grp, ok))) break;
+        if (!(ok = group_bar_and<kGroupWarps>(grp, ok))) break;
         if (wq == 0 && lane == 0)
             feed_stage(&full[grp * kGroupStages + q], smem_u32(sa), kKABytes, blk + kGroupStages * step, kKBM,
                        P.nblk, boxes);
@@ -282,7 +288,7 @@ dgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
 constexpr int kFBM = 128;
 constexpr int kFABytes = kFBM * kKK * 4;  // 32 KB per stage
 constexpr int kFBBytes = kKK * kKN * 4;   // 16 KB, resident
-constexpr size_t kFSmem = 1024 + (size_t)kGroups * kFABytes + kFBBytes + 256;
+constexpr size_t kFSmem = 1024 + (size_t)kFGroups * kFABytes + kFBBytes + 256;
 
 struct SkinnyParamsF {
     int M, N, K, nblk;
@@ -302,14 +308,14 @@ __global__ void __launch_bounds__(kKThreads, 1)
 sgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ SkinnyParamsF P) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    float* sB = reinterpret_cast<float*>(smem + kGroups * kFABytes);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kGroups * kFABytes + kFBBytes);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(full + kGroups);
+    float* sB = reinterpret_cast<float*>(smem + kFGroups * kFABytes);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kFGroups * kFABytes + kFBBytes);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(full + kFGroups);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int grp = warp / kGroupWarps, wq = warp % kGroupWarps;
+    const int grp = warp / kFGroupWarps, wq = warp % kFGroupWarps;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kGroups; ++s) mbar_init(&full[s], 1);
+        for (int s = 0; s < kFGroups; ++s) mbar_init(&full[s], 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -325,7 +331,7 @@ sgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             for (int b = 0; b < 2; ++b) tma_load_2d(st + b * 16384, &tmA, bar, 32 * b, i0);
         }
     };
-    const int step = kGroups * gridDim.x;
+    const int step = kFGroups * gridDim.x;
     int blk = blockIdx.x + grp * gridDim.x;
     if (wq == 0 && lane == 0) {
         prefetch_tmap(&tmA);
@@ -349,7 +355,7 @@ sgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
     __syncthreads();
 
-    const int u = threadIdx.x % (kGroupWarps * 32);
+    const int u = threadIdx.x % (kFGroupWarps * 32);
     const int tm = u & 15, tn = u >> 4;
     const bool busy = 8 * tn < P.N;
     uint32_t ph = 0;
@@ -403,7 +409,7 @@ sgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                 }
             }
         }
-        if (!(ok = group_bar_and(grp, ok))) break;
+        if (!(ok = group_bar_and<kFGroupWarps>(grp, ok))) break;
         ph ^= 1u;
         const int i0 = blk * kFBM;
         if (wq == 0 && lane == 0) feed_stage(&full[grp], smem_u32(sa), kFABytes, blk + step, kFBM, P.nblk, boxes);
