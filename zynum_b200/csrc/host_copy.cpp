@@ -13,7 +13,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
-#include <system_error>
+#include <exception>
 
 namespace zb {
 
@@ -73,18 +73,19 @@ bool CopyTeam::staged(const void* host, size_t width, size_t height) {
     const int want = std::min<int>(PinnedSlots::kThreads, (int)std::thread::hardware_concurrency() / 2);
     if (want < 2 || slots_.reserve() != cudaSuccess) return false;
     try {
+        threads_.reserve(want - 1);
         while ((int)threads_.size() < want - 1) {
             const int id = (int)threads_.size() + 1;
-            threads_.emplace_back([this, id] { loop(id); });
+            const long seen = generation_;  // no transfer is running: the first one it takes part in is the next
+            threads_.emplace_back([this, id, seen] { loop(id, seen); });
         }
-    } catch (const std::system_error&) {  // no more threads: those that started, and this one, do the work
+    } catch (const std::exception&) {  // no more threads: those that started, and this one, do the work
     }
     return true;
 }
 
-void CopyTeam::loop(int id) {
+void CopyTeam::loop(int id, long seen) {
     cudaSetDevice(device_);
-    long seen = 0;
     for (;;) {
         // the transfers of one call follow each other within microseconds: poll for the next
         // one for a while before sleeping (a wake-up costs 50 to 100 us here)

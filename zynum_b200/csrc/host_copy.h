@@ -54,7 +54,7 @@ class CopyTeam {
     bool staged(const void* host, size_t width, size_t height);
     cudaError_t run(Job j);
     void work(int id);
-    void loop(int id);
+    void loop(int id, long seen);
 
     PinnedSlots& slots_;
     int device_;
