@@ -30,7 +30,7 @@
 namespace zb {
 namespace {
 
-constexpr int kBK = 16;
+constexpr int kBK = kDgemmSlice;
 
 template <int ROWS, int COLS, int PITCH, int VEC, int NTHREADS>
 ZB_DEVICE void load_tile(double* smem, const double* __restrict__ base, long ld, int r0, int c0, int r_lim,
@@ -471,47 +471,13 @@ static bool use_tma_operands(const GemmArgsF64& g) {
     }();
     return enabled && dgemm_tma_applies(g);
 }
-static bool use_tma_tiles(const GemmArgsF64& g, const GemmPlan& plan) {
-    return plan.tile == TILE_128x128 && use_tma_operands(g);
-}
-
-// Cluster size with which a planned product runs on the 64 x 64 warp-specialised tiles
-// instead (dgemm_ws, which needs none of the plan's workspace); 0: it does not.
-static int ws_cluster(const GemmArgsF64& g, const GemmPlan& plan) {
-    if (!plan.automatic) return 0;
-    constexpr long sms = 148;
-    const long t64 = (long)((g.m + 63) / 64) * ((g.n + 63) / 64);
-    if (plan.tile == TILE_64x64) {
-        // about one 64 x 64 tile per SM: two CTAs of a cluster per tile.  Fewer tiles keep the
-        // cp.async tiles, which split K further and reduce through L2 (clusters of 4 and 8
-        // lost to them: 384 x 384 x 1024 21.0 against 15.5 us, 256 x 256 x 1024 15.3 / 9.3).
-        return 4 * t64 > 2 * sms && 2 * t64 <= 2 * sms && g.k >= 256 && use_tma_operands(g) ? 2 : 0;
-    }
-    if (plan.tile != TILE_128x128 || plan.splits > 1 || g.k < 256) return 0;
-    // both tile sizes run in rounds of one tile per SM; a 128 x 128 round at 0.955 of the
-    // pipe, a 64 x 64 one (a quarter of the work) at 0.90 (2048^3: 559 / 517 us, 3000^3 TT
-    // 1689 / 1628, 1536^3, one round of 128 x 128 tiles, 212 / 229)
-    const long m1 = (g.m + 127) / 128, n1 = (g.n + 127) / 128, m6 = (g.m + 63) / 64;
-    const long live1 = g.tri ? m1 * (m1 + 1) / 2 : m1 * n1, live6 = g.tri ? m6 * (m6 + 1) / 2 : t64;
-    const double r128 = 4.0 * ((live1 + sms - 1) / sms) / 0.955, r64 = ((live6 + sms - 1) / sms) / 0.90;
-    return r64 < 0.98 * r128 && use_tma_operands(g) ? 1 : 0;
-}
-
-// Cluster size with which a planned small product runs on the 64 x 64 cluster tiles
-// (dgemm_cluster_kernel: one launch, none of the plan's workspace); 0: it does not.
-static int small_cluster(const GemmArgsF64& g, const GemmPlan& plan) {
-    // up to two CTAs per SM, and no fewer K ranges than the workspace route has (which splits
-    // down to 64-deep slices: 256 x 256 x 1024 takes it 9.6 us, a cluster of 8 15.1)
-    const long t64 = (long)((g.m + 63) / 64) * ((g.n + 63) / 64);
-    if (!plan.automatic || plan.tile != TILE_64x64 || plan.splits < 2 || 4 * t64 > 2 * 148) return 0;
-    return g.k <= 256 || plan.splits == 4 ? 4 : 0;
-}
 
 int dgemm_native_used_splits(const GemmArgsF64& g, const GemmPlan& plan) {
     const int splits = plan.splits < 1 ? 1 : plan.splits;
     if (plan.tile == TILE_GEMV && gemv_applies(g.m, g.n, g.k, g.tri)) return gemv_used_splits(g.k, splits);
     if (skinny_gemm_applies(g.m, g.n, g.k, g.tri)) return 1;
-    int k_chunk = use_tma_tiles(g, plan) ? dgemm_tma_k_chunk(g.k, splits) : (g.k + splits - 1) / splits;
+    const bool tma = plan.tile == TILE_128x128 && use_tma_operands(g);
+    int k_chunk = tma ? dgemm_tma_k_chunk(g.k, splits) : (g.k + splits - 1) / splits;
     k_chunk = (k_chunk + kBK - 1) / kBK * kBK;
     return (g.k + k_chunk - 1) / k_chunk;
 }
@@ -530,12 +496,20 @@ cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* wor
     const bool aligned = ((reinterpret_cast<uintptr_t>(g.a) | reinterpret_cast<uintptr_t>(g.b)) % 16 == 0) &&
                          (g.lda % 2 == 0) && (g.ldb % 2 == 0);
     const int vec = aligned ? 2 : 1;
-    const int splits = plan.splits < 1 ? 1 : plan.splits;
-    int k_chunk = (g.k + splits - 1) / splits;
-    k_chunk = (k_chunk + kBK - 1) / kBK * kBK;
-    const int used = (g.k + k_chunk - 1) / k_chunk;
-    if (const int ws = ws_cluster(g, plan)) return dgemm_ws(g, ws, st);
-    if (const int c = small_cluster(g, plan)) return run_cluster(g, vec, c, st);
+    const DgemmRoute r = dgemm_tile_route(g.m, g.n, g.k, g.tri, use_tma_operands(g), plan);
+    const int used = r.ranges, k_chunk = r.k_chunk;
+    switch (r.kernel) {
+        case DGEMM_WS_64:
+            return dgemm_ws(g, r.cluster, st);
+        case DGEMM_CLUSTER_64:
+            return run_cluster(g, vec, r.cluster, st);
+        case DGEMM_TMA_128: {
+            const bool partials = used > 1 && r.cluster == 1;
+            if (partials && !workspace) return cudaErrorInvalidValue;
+            cudaError_t e = dgemm_tma(g, plan.splits, workspace, r.cluster > 1, st);
+            return e != cudaSuccess || !partials ? e : splitk_reduce(g, used, workspace, st);
+        }
+    }
     switch (plan.tile) {
         case TILE_128x64:
             return run_tiles<128, 64, 64, 32, 4>(g, vec, used, k_chunk, workspace, st);
@@ -546,15 +520,6 @@ cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* wor
         case TILE_64x64:  // few output tiles: 64 x 64 tiles, warps 2 x 2 of 32 x 32
             return run_tiles<64, 64, 32, 32, 4>(g, vec, used, k_chunk, workspace, st);
         default:
-            if (use_tma_tiles(g, plan)) {
-                const int kc = dgemm_tma_k_chunk(g.k, splits);
-                const int used_t = (g.k + kc - 1) / kc;
-                const bool cluster = used_t == 2 && plan.automatic;
-                if (used_t > 1 && !cluster && !workspace) return cudaErrorInvalidValue;
-                cudaError_t e = dgemm_tma(g, splits, workspace, cluster, st);
-                if (e != cudaSuccess || used_t == 1 || cluster) return e;
-                return splitk_reduce(g, used_t, workspace, st);
-            }
             // op(B) k-contiguous (transb N): three 32-deep stages (212 KB), half the block
             // barriers of 16-deep slices (+2 % measured at 2048-8192); otherwise four 16-deep
             // stages (32-deep slices measured 1 % slower there)

@@ -37,7 +37,7 @@
 namespace zb {
 namespace {
 
-constexpr int kTBM = 128, kTBN = 128, kTBK = 32, kTStages = 3;
+constexpr int kTBM = 128, kTBN = 128, kTBK = kDgemmTmaSlice, kTStages = 3;
 constexpr int kTMathWarps = 8;                     // 2 (M) x 4 (N) warps of 64 x 32
 constexpr int kTThreads = (kTMathWarps + 4) * 32;  // + a producer warpgroup (one TMA thread)
 // Register split: 384 threads launch with 168 registers each (64512); the
@@ -385,12 +385,6 @@ cudaError_t make_f64_map(CUtensorMap* map, const double* base, long inner, long 
 bool dgemm_tma_applies(const GemmArgsF64& g) {
     const uintptr_t bits = reinterpret_cast<uintptr_t>(g.a) | reinterpret_cast<uintptr_t>(g.b);
     return bits % 16 == 0 && g.lda % 2 == 0 && g.ldb % 2 == 0 && tensor_map_encoder() != nullptr;
-}
-
-int dgemm_tma_k_chunk(int k, int splits) {
-    splits = splits < 1 ? 1 : splits;
-    const int c = (k + splits - 1) / splits;
-    return (c + kTBK - 1) / kTBK * kTBK;
 }
 
 cudaError_t dgemm_tma(const GemmArgsF64& g, int splits, double* workspace, bool cluster, cudaStream_t st) {

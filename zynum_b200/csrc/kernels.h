@@ -66,7 +66,6 @@ cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* wor
 // z * m * n, ld m) and the caller reduces them; with `cluster`, exactly two ranges are
 // summed between the two CTAs of a cluster and no workspace is used.
 bool dgemm_tma_applies(const GemmArgsF64& g);
-int dgemm_tma_k_chunk(int k, int splits);
 cudaError_t dgemm_tma(const GemmArgsF64& g, int splits, double* workspace, bool cluster, cudaStream_t st);
 // Warp-specialised 64 x 64 DGEMM tiles (gemm_f64_ws.cu), K split over the CTAs of a
 // cluster of `splits` (1 or 2) that sum their partial tiles through distributed
@@ -146,5 +145,24 @@ void* tensor_map_encoder();
 
 // ---------------------------------------------------------------- planner
 GemmPlan plan_native_gemm(int m, int n, int k, int elem_bytes, int sm_count);
+
+constexpr int kDgemmSlice = 16, kDgemmTmaSlice = 32;  // depth of a K slice of the cp.async / TMA tiles
+int dgemm_tma_k_chunk(int k, int splits);
+
+// Kernels that run a product planned for tiles (not the matrix-vector and tall-skinny routes).
+enum DgemmKernel : int {
+    DGEMM_TILES = 0,       // cp.async tiles of the planned shape
+    DGEMM_TMA_128 = 1,     // TMA 128 x 128 tiles
+    DGEMM_WS_64 = 2,       // warp-specialised TMA 64 x 64 tiles
+    DGEMM_CLUSTER_64 = 3,  // cp.async 64 x 64 tiles in clusters
+};
+struct DgemmRoute {
+    int kernel = DGEMM_TILES;
+    int cluster = 1;  // CTAs that share a tile's K range and sum it between them
+    int ranges = 1;   // K ranges of k_chunk each (DGEMM_TILES, DGEMM_TMA_128)
+    int k_chunk = 0;
+};
+// `tma`: both operands can be described to TMA (dgemm_tma_applies).
+DgemmRoute dgemm_tile_route(int m, int n, int k, int tri, bool tma, const GemmPlan& plan);
 
 }  // namespace zb

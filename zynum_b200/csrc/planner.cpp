@@ -4,7 +4,8 @@
 // desiredThreadCount :88 / rowTaskCount :170 / runPlannedTasks :296 split C
 // into at most 64 disjoint column/row tasks for host threads.  On the GPU the
 // equivalent decision is how many CTAs cover C (tile shape) and, when C has
-// too few tiles to fill the 148 SMs, how far to split K.
+// too few tiles to fill the 148 SMs, how far to split K; dgemm_tile_route then
+// says which kernel runs the planned tiles.  Host code only.
 #include <algorithm>
 
 #include "kernels.h"
@@ -61,6 +62,78 @@ GemmPlan plan_native_gemm(int m, int n, int k, int elem_bytes, int sm_count) {
         if (s >= 2) p.splits = (int)s;
     }
     return p;
+}
+
+int dgemm_tma_k_chunk(int k, int splits) {
+    splits = std::max(1, splits);
+    const int c = (k + splits - 1) / splits;
+    return (c + kDgemmTmaSlice - 1) / kDgemmTmaSlice * kDgemmTmaSlice;
+}
+
+namespace {
+
+constexpr long kMaxGridY = 65535;  // the tile kernels put column tiles on grid.y
+
+// Cluster size with which a planned product runs on the 64 x 64 warp-specialised tiles
+// instead (dgemm_ws, which needs none of the plan's workspace); 0: it does not.
+int ws_cluster(int m, int n, int k, int tri, bool tma, const GemmPlan& plan) {
+    if (!plan.automatic) return 0;
+    constexpr long sms = 148;
+    const long t64 = (long)((m + 63) / 64) * ((n + 63) / 64);
+    if (plan.tile == TILE_64x64) {
+        // about one 64 x 64 tile per SM: two CTAs of a cluster per tile.  Fewer tiles keep the
+        // cp.async tiles, which split K further and reduce through L2 (clusters of 4 and 8
+        // lost to them: 384 x 384 x 1024 21.0 against 15.5 us, 256 x 256 x 1024 15.3 / 9.3).
+        return 4 * t64 > 2 * sms && 2 * t64 <= 2 * sms && k >= 256 && tma ? 2 : 0;
+    }
+    if (plan.tile != TILE_128x128 || plan.splits > 1 || k < 256) return 0;
+    // 64-wide column tiles run out of grid.y at half the columns of 128-wide ones
+    if ((n + 63L) / 64 > kMaxGridY) return 0;
+    // both tile sizes run in rounds of one tile per SM; a 128 x 128 round at 0.955 of the
+    // pipe, a 64 x 64 one (a quarter of the work) at 0.90 (2048^3: 559 / 517 us, 3000^3 TT
+    // 1689 / 1628, 1536^3, one round of 128 x 128 tiles, 212 / 229)
+    const long m1 = (m + 127) / 128, n1 = (n + 127) / 128, m6 = (m + 63) / 64;
+    const long live1 = tri ? m1 * (m1 + 1) / 2 : m1 * n1, live6 = tri ? m6 * (m6 + 1) / 2 : t64;
+    const double r128 = 4.0 * ((live1 + sms - 1) / sms) / 0.955, r64 = ((live6 + sms - 1) / sms) / 0.90;
+    return r64 < 0.98 * r128 && tma ? 1 : 0;
+}
+
+// Cluster size with which a planned small product runs on the 64 x 64 cluster tiles
+// (dgemm_cluster_kernel: one launch, none of the plan's workspace); 0: it does not.
+int small_cluster(int m, int n, int k, const GemmPlan& plan) {
+    // up to two CTAs per SM, and no fewer K ranges than the workspace route has (which splits
+    // down to 64-deep slices: 256 x 256 x 1024 takes it 9.6 us, a cluster of 8 15.1)
+    const long t64 = (long)((m + 63) / 64) * ((n + 63) / 64);
+    if (!plan.automatic || plan.tile != TILE_64x64 || plan.splits < 2 || 4 * t64 > 2 * 148) return 0;
+    return k <= 256 || plan.splits == 4 ? 4 : 0;
+}
+
+}  // namespace
+
+DgemmRoute dgemm_tile_route(int m, int n, int k, int tri, bool tma, const GemmPlan& plan) {
+    DgemmRoute r;
+    const int splits = std::max(1, plan.splits);
+    if (const int c = ws_cluster(m, n, k, tri, tma, plan)) {
+        r.kernel = DGEMM_WS_64;
+        r.cluster = c;
+        return r;
+    }
+    if (const int c = small_cluster(m, n, k, plan)) {
+        r.kernel = DGEMM_CLUSTER_64;
+        r.cluster = c;
+        return r;
+    }
+    if (plan.tile == TILE_128x128 && tma) {
+        r.kernel = DGEMM_TMA_128;
+        r.k_chunk = dgemm_tma_k_chunk(k, splits);
+        r.ranges = (k + r.k_chunk - 1) / r.k_chunk;
+        if (r.ranges == 2 && plan.automatic) r.cluster = 2;
+        return r;
+    }
+    r.kernel = DGEMM_TILES;
+    r.k_chunk = ((k + splits - 1) / splits + kDgemmSlice - 1) / kDgemmSlice * kDgemmSlice;
+    r.ranges = (k + r.k_chunk - 1) / r.k_chunk;
+    return r;
 }
 
 }  // namespace zb
