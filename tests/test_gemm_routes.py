@@ -1,9 +1,11 @@
 """Routing rules of the native GEMM kernels (host code, no GPU)."""
 from __future__ import annotations
 
+import itertools
+
 import pytest
 
-from gemm_routes import CLUSTER_64, TMA_128, WS_64, dgemm_route
+from gemm_routes import CLUSTER_64, TILES, TMA_128, WS_64, dgemm_route
 
 MAX_GRID_Y = 65535
 TILE_COLS = {TMA_128: 128, WS_64: 64, CLUSTER_64: 64}
@@ -21,3 +23,26 @@ def test_column_tiles_fit_the_grid(m, n, k):
 def test_last_column_count_of_the_64_wide_tiles():
     assert dgemm_route(64, 64 * MAX_GRID_Y, 256).kernel == WS_64
     assert dgemm_route(64, 64 * MAX_GRID_Y + 1, 256).kernel == TMA_128
+
+
+@pytest.mark.parametrize("tma", [True, False])
+@pytest.mark.parametrize("tri", [0, 1])
+def test_clusters_keep_the_planned_k_ranges(tma, tri):
+    """A cluster adds up K ranges no longer than those the plan would sum through the
+    workspace: longer ones round worse, and leave SMs idle (576 x 576 x 1024)."""
+    sizes = [17, 64, 65, 128, 250, 320, 384, 512, 576, 640, 704, 770, 1000, 1024]
+    for m, n, k in itertools.product(sizes, sizes, [64, 128, 200, 256, 300, 512, 777, 1024, 1025, 2000, 4096]):
+        if tri and m != n:
+            continue
+        r, planned = dgemm_route(m, n, k, tri, tma), dgemm_route(m, n, k, tri, tma, automatic=False)
+        chunk = r.k_chunk
+        if r.kernel in (WS_64, CLUSTER_64):
+            chunk = ((k + r.cluster - 1) // r.cluster + 15) // 16 * 16
+        assert min(k, chunk) <= min(k, planned.k_chunk), (m, n, k, r, planned)
+
+
+def test_cluster_of_two_range():
+    assert dgemm_route(576, 576, 1024).kernel == TILES  # 81 tiles, three ranges
+    assert dgemm_route(576, 704, 1024)[2:4] == (WS_64, 2)  # 99 tiles, two ranges
+    assert dgemm_route(1024, 512, 512)[2:4] == (WS_64, 2)
+    assert dgemm_route(768, 768, 512)[2:4] == (WS_64, 2)  # 144 tiles

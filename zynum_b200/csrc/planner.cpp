@@ -81,10 +81,13 @@ int ws_cluster(int m, int n, int k, int tri, bool tma, const GemmPlan& plan) {
     constexpr long sms = 148;
     const long t64 = (long)((m + 63) / 64) * ((n + 63) / 64);
     if (plan.tile == TILE_64x64) {
-        // about one 64 x 64 tile per SM: two CTAs of a cluster per tile.  Fewer tiles keep the
-        // cp.async tiles, which split K further and reduce through L2 (clusters of 4 and 8
-        // lost to them: 384 x 384 x 1024 21.0 against 15.5 us, 256 x 256 x 1024 15.3 / 9.3).
-        return 4 * t64 > 2 * sms && 2 * t64 <= 2 * sms && k >= 256 && tma ? 2 : 0;
+        // about one 64 x 64 tile per SM (99 .. 148 tiles on 148 SMs), which is where the plan has
+        // two K ranges: two CTAs of a cluster per tile.  Fewer tiles keep the cp.async tiles,
+        // which split K further and reduce through L2 (81 tiles, three ranges against a cluster
+        // of two: 576 x 576 x 1024 34.5 against 44.9 us, and two ranges round worse than three;
+        // clusters of 4 and 8 lost too: 384 x 384 x 1024 21.0 / 15.5 us, 256 x 256 x 1024 15.3 /
+        // 9.3).  110 tiles, 640 x 704 x 512: 26.3 us on the cluster, 29.1 through the workspace.
+        return plan.splits == 2 && k >= 256 && tma ? 2 : 0;
     }
     if (plan.tile != TILE_128x128 || plan.splits > 1 || k < 256) return 0;
     // 64-wide column tiles run out of grid.y at half the columns of 128-wide ones
