@@ -15,3 +15,10 @@ extern "C" void dgemm_route(int m, int n, int k, int tri, int tma, int automatic
     const int v[6] = {p.tile, p.splits, r.kernel, r.cluster, r.ranges, r.k_chunk};
     for (int i = 0; i < 6; ++i) out[i] = v[i];
 }
+
+// out: planned splits, cluster, halves
+extern "C" void sgemm_route(int m, int n, int k, int sms, int* out) {
+    const zb::GemmPlan p = zb::plan_native_gemm(m, n, k, 4, sms);
+    const zb::SgemmRoute r = zb::sgemm_tile_route(m, n, k, p);
+    out[0] = p.splits, out[1] = r.cluster, out[2] = r.halves;
+}

@@ -16,6 +16,7 @@ TILE_128x128, TILE_64x64 = 0, 5
 TILES, TMA_128, WS_64, CLUSTER_64 = range(4)
 
 Route = namedtuple("Route", "tile splits kernel cluster ranges k_chunk")
+SgemmRoute = namedtuple("SgemmRoute", "splits cluster halves")
 
 
 @functools.lru_cache(maxsize=None)
@@ -32,3 +33,9 @@ def dgemm_route(m, n, k, tri=0, tma=True, automatic=True, sms=148):
     out = (C.c_int * 6)()
     _shim().dgemm_route(m, n, k, tri, int(tma), int(automatic), sms, out)
     return Route(*out)
+
+
+def sgemm_route(m, n, k, sms=148):
+    out = (C.c_int * 3)()
+    _shim().sgemm_route(m, n, k, sms, out)
+    return SgemmRoute(*out)

@@ -5,7 +5,7 @@ import itertools
 
 import pytest
 
-from gemm_routes import CLUSTER_64, TILES, TMA_128, WS_64, dgemm_route
+from gemm_routes import CLUSTER_64, TILES, TMA_128, WS_64, dgemm_route, sgemm_route
 
 MAX_GRID_Y = 65535
 TILE_COLS = {TMA_128: 128, WS_64: 64, CLUSTER_64: 64}
@@ -46,3 +46,21 @@ def test_cluster_of_two_range():
     assert dgemm_route(576, 704, 1024)[2:4] == (WS_64, 2)  # 99 tiles, two ranges
     assert dgemm_route(1024, 512, 512)[2:4] == (WS_64, 2)
     assert dgemm_route(768, 768, 512)[2:4] == (WS_64, 2)  # 144 tiles
+
+
+def test_sgemm_clusters_keep_the_planned_k_ranges():
+    """As above for FP32: 128 x 64 cluster tiles (16-deep slices) against the plan's 128 x 128
+    tiles, whose ranges are multiples of 32."""
+    up = lambda x, q: (x + q - 1) // q * q  # noqa: E731
+    sizes = [17, 64, 128, 129, 256, 300, 384, 512, 600, 640, 900, 1024, 2000, 4096]
+    clusters = set()
+    for m, n, k in itertools.product(sizes, sizes, [16, 100, 256, 511, 512, 801, 1000, 1300, 2048, 2310, 2560, 4000]):
+        r = sgemm_route(m, n, k)
+        if not r.cluster:
+            continue
+        chunk = up(up(k, r.cluster) // r.cluster, 16)
+        if r.halves:
+            chunk = (chunk // 16 + 1) // 2 * 16
+        assert min(k, chunk) <= min(k, up(up(k, r.splits) // r.splits, 32)), (m, n, k, r)
+        clusters.add(r[1:])
+    assert clusters == {(8, 0), (4, 0), (2, 0), (1, 0), (8, 1), (4, 1), (2, 1)}

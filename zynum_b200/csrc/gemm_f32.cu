@@ -125,8 +125,8 @@ ZB_DEVICE void unpack_f32x2(uint64_t v, float& x, float& y) {
 // Thread (tx, ty) owns rows {ty*4 + i, 64 + ty*4 + i} and columns
 // {64 q + tx*4 + j}, q < BN / 64; a warp covers 4 ty x 8 tx, so each float4
 // fragment load touches 4 (A) or 8 (B) distinct 16-byte words: one
-// shared-memory wavefront.
-template <bool A_MNFAST, bool B_MNFAST, int VEC, int BN>
+// shared-memory wavefront.  HALVES: the range's two halves are summed apart and added.
+template <bool A_MNFAST, bool B_MNFAST, int VEC, int BN, bool HALVES = false>
 ZB_DEVICE void sgemm_products(float (&acc)[8][BN / 16], float* smf, int M, int N, int m0, int n0, int kb, int ke,
                               const float* __restrict__ A, long lda, const float* __restrict__ B, long ldb) {
     constexpr int BK = Cfg<BN>::BK, STAGES = Cfg<BN>::STAGES, JN = BN / 16, PA = pitch(kBM), PB = pitch(BN);
@@ -141,11 +141,14 @@ ZB_DEVICE void sgemm_products(float (&acc)[8][BN / 16], float* smf, int M, int N
     const uint32_t a_valid = LA::init(m0, M), b_valid = LB::init(n0, N);
 
     // acc2[p][j]: rows (2p, 2p + 1) of the thread's eight and column j, as one packed pair
-    uint64_t acc2[4][JN];
+    uint64_t acc2[4][JN], first[HALVES ? 4 : 1][HALVES ? JN : 1];
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
-        for (int j = 0; j < JN; ++j) acc2[p][j] = 0ull;
+        for (int j = 0; j < JN; ++j) {
+            acc2[p][j] = 0ull;
+            if constexpr (HALVES) first[p][j] = 0ull;
+        }
 
     auto load_stage = [&](int stage, int kt) {
         const int k0 = kb + kt * BK;
@@ -191,12 +194,31 @@ ZB_DEVICE void sgemm_products(float (&acc)[8][BN / 16], float* smf, int M, int N
                 for (int p = 0; p < 4; ++p) fma_f32x2(acc2[p][j], a2[p], bb);
             }
         }
+        if constexpr (HALVES) {
+            if (kt + 1 == (KT + 1) / 2) {
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+#pragma unroll
+                    for (int j = 0; j < JN; ++j) {
+                        first[p][j] = acc2[p][j];
+                        acc2[p][j] = 0ull;
+                    }
+            }
+        }
     }
     cp_async_wait<0>();
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
-        for (int j = 0; j < JN; ++j) unpack_f32x2(acc2[p][j], acc[2 * p][j], acc[2 * p + 1][j]);
+        for (int j = 0; j < JN; ++j) {
+            unpack_f32x2(acc2[p][j], acc[2 * p][j], acc[2 * p + 1][j]);
+            if constexpr (HALVES) {
+                float x, y;
+                unpack_f32x2(first[p][j], x, y);
+                acc[2 * p][j] += x;
+                acc[2 * p + 1][j] += y;
+            }
+        }
 }
 
 template <bool A_MNFAST, bool B_MNFAST, int VEC, bool PARTIAL, int BN>
@@ -275,10 +297,14 @@ sgemm_ffma_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __
 // Bound: latency and the share of the SMs a small product can use; 128 x 128 tiles with
 // slices of at least 256 left most of them idle (512^3: 32 CTAs).  512^3 34.6 -> 12.3 us,
 // 256^3 31.0 -> 6.3, 128^3 15.8 -> 5.6, 64 x 2000 x 100 TT 15.8 -> 8.0.
+// HALVES (the plan has more K ranges than the cluster CTAs): a CTA sums the halves of its
+// range apart, so that no sum is longer than the plan's and rounds worse (300 x 300 x 4000,
+// 8 CTAs against 15 ranges: rms error 0.110 u on the plan, 0.143 on whole ranges, 0.103 in
+// halves, both 39.1 us).
 constexpr int kCN = 64, kCPitch = kBM + 4;
 
-template <bool A_MNFAST, bool B_MNFAST, int VEC>
-__global__ void __launch_bounds__(kThreads, Cfg<kCN>::MINB)
+template <bool A_MNFAST, bool B_MNFAST, int VEC, bool HALVES>
+__global__ void __launch_bounds__(kThreads, HALVES ? 2 : Cfg<kCN>::MINB)
 sgemm_cluster_kernel(int M, int N, int K, int k_chunk, float alpha, const float* __restrict__ A, long lda,
                      const float* __restrict__ B, long ldb, float beta, float* __restrict__ C, long ldc, int tri) {
     constexpr int JN = kCN / 16;
@@ -291,7 +317,7 @@ sgemm_cluster_kernel(int M, int N, int K, int k_chunk, float alpha, const float*
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tx = (warp & 1) * 8 + (lane & 7), ty = (warp >> 1) * 4 + (lane >> 3);
     float acc[8][JN];
-    sgemm_products<A_MNFAST, B_MNFAST, VEC, kCN>(acc, smf, M, N, m0, n0, kb, ke, A, lda, B, ldb);
+    sgemm_products<A_MNFAST, B_MNFAST, VEC, kCN, HALVES>(acc, smf, M, N, m0, n0, kb, ke, A, lda, B, ldb);
     __syncthreads();  // the ring becomes the partial tile [column][row]
 #pragma unroll
     for (int j = 0; j < JN; ++j)
@@ -364,11 +390,11 @@ cudaError_t launch_f32(const GemmArgsF32& g, int splits, int k_chunk, float* W, 
     return cudaGetLastError();
 }
 
-template <bool AM, bool BM_, int VEC>
+template <bool AM, bool BM_, int VEC, bool HALVES>
 cudaError_t launch_cluster_f32(const GemmArgsF32& g, int splits, cudaStream_t st) {
     constexpr size_t SMEM = (size_t)Cfg<kCN>::STAGES * Cfg<kCN>::BK * (pitch(kBM) + pitch(kCN)) * sizeof(float);
     static_assert(SMEM >= (size_t)kCN * kCPitch * sizeof(float), "the partial tile reuses the ring");
-    auto kern = sgemm_cluster_kernel<AM, BM_, VEC>;
+    auto kern = sgemm_cluster_kernel<AM, BM_, VEC, HALVES>;
     cudaError_t e = ensure_dynamic_smem(kern, (int)SMEM);
     if (e != cudaSuccess) return e;
     const int k_chunk = ((g.k + splits - 1) / splits + 15) / 16 * 16;
@@ -393,26 +419,15 @@ cudaError_t launch_cluster_f32(const GemmArgsF32& g, int splits, cudaStream_t st
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// Cluster size of the 128 x 64 cluster tiles for a product planned with `splits` K ranges of
-// 128 x 128 tiles; 0: it keeps the plan.  The largest cluster with at most one CTA per SM and
-// 16-deep ranges, where its CTAs then have less to do than the plan's: (K / c) x 64 columns
-// against (K / splits) x 128 (1024^3: c = 1 against two K ranges, 65 against 61 us, keeps the plan;
-// 300 x 300 x 4000, c = 8 against 15: 36.9 / 37.1; 256 x 256 x 262144, c = 8 against 37, keeps it).
-int cluster_splits(const GemmArgsF32& g, int splits) {
-    const long t = (long)((g.m + kBM - 1) / kBM) * ((g.n + kCN - 1) / kCN);
-    for (int c = 8; c >= 1; c /= 2)
-        if (c * t <= 148 && (c == 1 || g.k >= 16 * c)) return 2 * c > splits ? c : 0;
-    return 0;
-}
-
+template <bool HALVES>
 cudaError_t dispatch_cluster_f32(const GemmArgsF32& g, int vec, int splits, cudaStream_t st) {
     const bool am = g.transa == 'N', bm = g.transb != 'N';
 #define ZB_CASE(AM, BMF, V) \
-    if (am == AM && bm == BMF && vec == V) return launch_cluster_f32<AM, BMF, V>(g, splits, st);
+    if (am == AM && bm == BMF && vec == V) return launch_cluster_f32<AM, BMF, V, HALVES>(g, splits, st);
     ZB_CASE(false, true, 1) ZB_CASE(true, false, 1) ZB_CASE(true, true, 1)
     ZB_CASE(false, true, 4) ZB_CASE(true, false, 4) ZB_CASE(true, true, 4)
 #undef ZB_CASE
-    return launch_cluster_f32<false, false, 1>(g, splits, st);
+    return launch_cluster_f32<false, false, 1, HALVES>(g, splits, st);
 }
 
 template <bool PARTIAL>
@@ -551,7 +566,10 @@ cudaError_t sgemm_native(const GemmArgsF32& g_in, const GemmPlan& plan, float* w
     if (g.transb != 'N') aligned = aligned && (reinterpret_cast<uintptr_t>(g.b) % 16 == 0) && (g.ldb % 4 == 0);
     const int vec = aligned ? 4 : 1;
     const int splits = plan.splits < 1 ? 1 : plan.splits;
-    if (const int c = cluster_splits(g, splits)) return dispatch_cluster_f32(g, vec, c, st);
+    const SgemmRoute route = sgemm_tile_route(g.m, g.n, g.k, plan);
+    if (route.cluster)
+        return route.halves ? dispatch_cluster_f32<true>(g, vec, route.cluster, st)
+                            : dispatch_cluster_f32<false>(g, vec, route.cluster, st);
     int k_chunk = (g.k + splits - 1) / splits;
     k_chunk = (k_chunk + 31) / 32 * 32;  // a multiple of every BK
     const int used = (g.k + k_chunk - 1) / k_chunk;

@@ -165,4 +165,12 @@ struct DgemmRoute {
 // `tma`: both operands can be described to TMA (dgemm_tma_applies).
 DgemmRoute dgemm_tile_route(int m, int n, int k, int tri, bool tma, const GemmPlan& plan);
 
+// FP32 product planned for 128 x 128 tiles: cluster of the 128 x 64 cluster tiles (0: it keeps
+// the plan), each CTA's K range summed in two halves or as a whole.
+struct SgemmRoute {
+    int cluster = 0;
+    bool halves = false;
+};
+SgemmRoute sgemm_tile_route(int m, int n, int k, const GemmPlan& plan);
+
 }  // namespace zb

@@ -139,4 +139,21 @@ DgemmRoute dgemm_tile_route(int m, int n, int k, int tri, bool tma, const GemmPl
     return r;
 }
 
+// The largest cluster with at most one CTA per SM and 16-deep ranges, where its CTAs then have
+// less to do than the plan's: (K / c) x 64 columns against (K / splits) x 128 (1024^3: c = 1
+// against two K ranges, 65 against 61 us, keeps the plan; 300 x 300 x 4000, c = 8 against 15:
+// 36.9 / 37.1; 256 x 256 x 262144, c = 8 against 37, keeps it).
+SgemmRoute sgemm_tile_route(int m, int n, int k, const GemmPlan& plan) {
+    SgemmRoute r;
+    const int splits = std::max(1, plan.splits);
+    const long t = (long)((m + 127) / 128) * ((n + 63) / 64);
+    for (int c = 8; c >= 1; c /= 2)
+        if (c * t <= 148 && (c == 1 || k >= 16 * c)) {
+            r.cluster = 2 * c > splits ? c : 0;
+            r.halves = r.cluster && c < splits;
+            break;
+        }
+    return r;
+}
+
 }  // namespace zb
