@@ -64,3 +64,13 @@ def test_sgemm_clusters_keep_the_planned_k_ranges():
         assert min(k, chunk) <= min(k, up(up(k, r.splits) // r.splits, 32)), (m, n, k, r)
         clusters.add(r[1:])
     assert clusters == {(8, 0), (4, 0), (2, 0), (1, 0), (8, 1), (4, 1), (2, 1)}
+
+
+def test_cluster_routes_need_no_workspace():
+    for shape, route in (((256, 256, 256), (CLUSTER_64, 4)), ((1024, 512, 512), (WS_64, 2)),
+                         ((2048, 2048, 2048), (WS_64, 1)), ((2048, 512, 2048), (TMA_128, 2))):
+        r = dgemm_route(*shape)
+        assert r[2:4] == route and r.ranges == 1, (shape, r)
+    assert dgemm_route(256, 256, 4096).ranges == dgemm_route(256, 256, 4096, tma=False).ranges == 16
+    # a split count that the caller asked for keeps the workspace
+    assert dgemm_route(2048, 512, 2048, automatic=False).ranges == 2

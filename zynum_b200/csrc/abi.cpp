@@ -92,6 +92,14 @@ cudaError_t scale_matrix<float>(int m, int n, float beta, float* c, long ldc, cu
     return scale_matrix_f32(m, n, beta, c, ldc, st);
 }
 
+// Scratch the native kernels use for exactly this product.
+size_t native_workspace_bytes(const GemmArgsF64& g, const GemmPlan& p) {
+    return splitk_workspace_elems(g.m, g.n, dgemm_native_used_splits(g, p)) * sizeof(double);
+}
+size_t native_workspace_bytes(const GemmArgsF32& g, const GemmPlan& p) {
+    return sgemm_native_workspace_bytes(g.transa, g.transb, g.m, g.n, g.k, p);
+}
+
 // Device-pointer real GEMM on `st`; arguments already validated, m, n > 0.
 template <typename Scratch>
 cudaError_t run_dgemm(const GemmArgsF64& g, cudaStream_t st, Scratch scratch) {
@@ -109,7 +117,7 @@ cudaError_t run_dgemm(const GemmArgsF64& g, cudaStream_t st, Scratch scratch) {
     }
     GemmPlan p = plan_native_gemm(g.m, g.n, g.k, 8, cx.sm_count);
     void* ws = nullptr;
-    size_t need = splitk_workspace_elems(g.m, g.n, p.splits) * sizeof(double);
+    const size_t need = native_workspace_bytes(g, p);
     if (need) {
         cudaError_t e = scratch(need, st, &ws);
         if (e != cudaSuccess) return e;
@@ -145,7 +153,7 @@ cudaError_t run_sgemm(const GemmArgsF32& g, cudaStream_t st, Scratch scratch) {
     }
     GemmPlan p = plan_native_gemm(g.m, g.n, g.k, 4, cx.sm_count);
     void* ws = nullptr;
-    size_t need = sgemm_native_workspace_bytes(g.transa, g.transb, g.m, g.n, g.k, p);
+    const size_t need = native_workspace_bytes(g, p);
     if (need) {
         cudaError_t e = scratch(need, st, &ws);
         if (e != cudaSuccess) return e;
@@ -343,7 +351,7 @@ void host_gemm(const char* routine, char ta, char tb, int m, int n, int k, T alp
 }
 
 // ---------------------------------------------------------------- complex
-// Scratch the real GEMM of run_dgemm / run_sgemm would request for this shape.
+// The most scratch the real GEMM of run_dgemm / run_sgemm requests for this shape.
 size_t real_scratch_bytes(int m, int n, int k, double*) {
     Context& cx = context();
     int method = cx.dgemm_method;
@@ -633,8 +641,7 @@ cudaError_t run_syrk(char uplo, char trans, int n, int k, T alpha, const T* a, l
     g.tri = (uplo == 'U') ? 1 : 2;
     GemmPlan p = plan_native_gemm(n, n, k, sizeof(T), cx.sm_count);
     void* ws = nullptr;
-    const size_t need = sizeof(T) == 4 ? sgemm_native_workspace_bytes(g.transa, g.transb, n, n, k, p)
-                                       : splitk_workspace_elems(n, n, p.splits) * sizeof(T);
+    const size_t need = native_workspace_bytes(g, p);
     if (need) {
         cudaError_t e = scratch(need, st, &ws);
         if (e != cudaSuccess) return e;
@@ -691,8 +698,7 @@ cudaError_t run_syr2k(char uplo, char trans, int n, int k, T alpha, const T* a, 
     g1.tri = g2.tri = (uplo == 'U') ? 1 : 2;
     GemmPlan p = plan_native_gemm(n, n, k, sizeof(T), cx.sm_count);
     void* ws = nullptr;
-    const size_t need = sizeof(T) == 4 ? sgemm_native_workspace_bytes(t1, t2, n, n, k, p)
-                                       : splitk_workspace_elems(n, n, p.splits) * sizeof(T);
+    const size_t need = native_workspace_bytes(g1, p);  // the same for g2
     if (need) {
         cudaError_t e = scratch(need, st, &ws);
         if (e != cudaSuccess) return e;
@@ -1972,7 +1978,7 @@ int zynum_blas_gpu_dgemmt_device(char uplo, char transa, char transb, int n, int
     if (k == 0) return cuda_status(syrk_scale_only<double>(n, ul, beta, c, ldc, st), "dgemmt_device");
     GemmPlan p = plan_native_gemm(n, n, k, 8, cx.sm_count);
     void* ws = nullptr;
-    const size_t need = splitk_workspace_elems(n, n, p.splits) * sizeof(double);
+    const size_t need = native_workspace_bytes(g, p);
     if (need && (e = cx.stream_scratch(st, need, &ws)) != cudaSuccess) return cuda_status(e, "dgemmt_device");
     return cuda_status(dgemm_native(g, p, static_cast<double*>(ws), st), "dgemmt_device");
 }

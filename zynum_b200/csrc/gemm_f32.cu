@@ -496,12 +496,13 @@ struct Relayout {
 
 Relayout relayout_plan(char transa, char transb, int m, int n, int k, const GemmPlan& plan) {
     Relayout r;
-    r.splitk = align_elems(splitk_workspace_elems(m, n, plan.splits));
+    const bool tiles = plan.tile == TILE_128x128;
+    if (!tiles || !sgemm_tile_route(m, n, k, plan).cluster)  // a cluster sums its ranges itself
+        r.splitk = align_elems(splitk_workspace_elems(m, n, plan.splits));
     // the matrix-vector, narrow and tall-skinny kernels read either layout directly (the
     // tall-skinny route, K <= 64, never splits K either, so it needs no workspace at all,
     // e.g. on a stream under graph capture)
-    if (plan.tile == TILE_GEMV || plan.tile == TILE_NARROW_N || plan.tile == TILE_NARROW_M ||
-        skinny_gemm_applies(m, n, k, 0))
+    if (!tiles || skinny_gemm_applies(m, n, k, 0))
         return r;
     const size_t a_elems = align_elems((size_t)pad4(m) * (size_t)k);
     const size_t b_elems = align_elems((size_t)pad4(n) * (size_t)k);

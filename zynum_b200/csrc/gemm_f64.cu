@@ -476,14 +476,11 @@ int dgemm_native_used_splits(const GemmArgsF64& g, const GemmPlan& plan) {
     const int splits = plan.splits < 1 ? 1 : plan.splits;
     if (plan.tile == TILE_GEMV && gemv_applies(g.m, g.n, g.k, g.tri)) return gemv_used_splits(g.k, splits);
     if (skinny_gemm_applies(g.m, g.n, g.k, g.tri)) return 1;
-    const bool tma = plan.tile == TILE_128x128 && use_tma_operands(g);
-    int k_chunk = tma ? dgemm_tma_k_chunk(g.k, splits) : (g.k + splits - 1) / splits;
-    k_chunk = (k_chunk + kBK - 1) / kBK * kBK;
-    return (g.k + k_chunk - 1) / k_chunk;
+    return dgemm_tile_route(g.m, g.n, g.k, g.tri, use_tma_operands(g), plan).ranges;
 }
 
-// Entry used by the planner: `tile` selects the block shape, `splits` > 1
-// requires a workspace of splits * m * n doubles.
+// Entry used by the planner: `tile` selects the block shape; more than one range
+// (dgemm_native_used_splits) requires a workspace of that many times m * n doubles.
 cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* workspace, cudaStream_t st) {
     if (plan.tile == TILE_GEMV && gemv_applies(g.m, g.n, g.k, g.tri)) return dgemv_route(g, plan.splits, workspace, st);
     if (skinny_gemm_applies(g.m, g.n, g.k, g.tri)) {
@@ -504,10 +501,9 @@ cudaError_t dgemm_native(const GemmArgsF64& g, const GemmPlan& plan, double* wor
         case DGEMM_CLUSTER_64:
             return run_cluster(g, vec, r.cluster, st);
         case DGEMM_TMA_128: {
-            const bool partials = used > 1 && r.cluster == 1;
-            if (partials && !workspace) return cudaErrorInvalidValue;
+            if (used > 1 && !workspace) return cudaErrorInvalidValue;
             cudaError_t e = dgemm_tma(g, plan.splits, workspace, r.cluster > 1, st);
-            return e != cudaSuccess || !partials ? e : splitk_reduce(g, used, workspace, st);
+            return e != cudaSuccess || used == 1 ? e : splitk_reduce(g, used, workspace, st);
         }
     }
     switch (plan.tile) {

@@ -71,13 +71,13 @@ cudaError_t dgemm_tma(const GemmArgsF64& g, int splits, double* workspace, bool 
 // cluster of `splits` (1 or 2) that sum their partial tiles through distributed
 // shared memory: no workspace.  Needs dgemm_tma_applies(g).
 cudaError_t dgemm_ws(const GemmArgsF64& g, int splits, cudaStream_t st);
-// K ranges dgemm_native will actually use for this plan (1: no workspace); the
-// route (GEMV, tall-skinny, tiles) and the rounding of K slices can only lower
-// it below plan.splits.
+// K ranges whose sums dgemm_native will put into the workspace for this plan (1: it
+// needs none); the route (GEMV, tall-skinny, clusters that sum their ranges
+// themselves) and the rounding of K slices can only lower it below plan.splits.
 int dgemm_native_used_splits(const GemmArgsF64& g, const GemmPlan& plan);
 cudaError_t sgemm_native(const GemmArgsF32& g, const GemmPlan& plan, float* workspace, cudaStream_t st);
-// Workspace of sgemm_native in bytes: split-K partials plus, for large
-// products, an MN-contiguous copy of each K-contiguous operand.  The bound
+// Workspace of sgemm_native in bytes: split-K partials (none on the cluster
+// tiles) plus, for large products, an MN-contiguous copy of each K-contiguous operand.  The bound
 // covers every FP32 product of shape up to m x n x k and any transposes.
 size_t sgemm_native_workspace_bytes(char transa, char transb, int m, int n, int k, const GemmPlan& plan);
 // Tall-skinny route (n <= 64, k <= 64, m >= 2048, no triangle mode): op(B)
@@ -159,8 +159,8 @@ enum DgemmKernel : int {
 struct DgemmRoute {
     int kernel = DGEMM_TILES;
     int cluster = 1;  // CTAs that share a tile's K range and sum it between them
-    int ranges = 1;   // K ranges of k_chunk each (DGEMM_TILES, DGEMM_TMA_128)
-    int k_chunk = 0;
+    int ranges = 1;   // K ranges whose sums go through the workspace (1: none is needed)
+    int k_chunk = 0;  // depth of a K range (DGEMM_TILES, DGEMM_TMA_128)
 };
 // `tma`: both operands can be described to TMA (dgemm_tma_applies).
 DgemmRoute dgemm_tile_route(int m, int n, int k, int tri, bool tma, const GemmPlan& plan);

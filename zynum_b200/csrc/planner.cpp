@@ -130,7 +130,10 @@ DgemmRoute dgemm_tile_route(int m, int n, int k, int tri, bool tma, const GemmPl
         r.kernel = DGEMM_TMA_128;
         r.k_chunk = dgemm_tma_k_chunk(k, splits);
         r.ranges = (k + r.k_chunk - 1) / r.k_chunk;
-        if (r.ranges == 2 && plan.automatic) r.cluster = 2;
+        if (r.ranges == 2 && plan.automatic) {
+            r.cluster = 2;
+            r.ranges = 1;
+        }
         return r;
     }
     r.kernel = DGEMM_TILES;
