@@ -74,3 +74,16 @@ def test_cluster_routes_need_no_workspace():
     assert dgemm_route(256, 256, 4096).ranges == dgemm_route(256, 256, 4096, tma=False).ranges == 16
     # a split count that the caller asked for keeps the workspace
     assert dgemm_route(2048, 512, 2048, automatic=False).ranges == 2
+
+
+def test_rules_follow_the_sm_count():
+    """The routing rules use the SM count that the plan was made for (a partitioned GPU has fewer)."""
+    # up to two CTAs per SM: 49 tiles in clusters of four are 196 CTAs
+    assert dgemm_route(400, 400, 200, sms=148).kernel == CLUSTER_64
+    assert dgemm_route(400, 400, 200, sms=74).kernel == TILES
+    # rounds of tiles: 121 tiles of 128 x 128 are one round on 148 SMs, two on 74 (484 of 64 x 64: seven)
+    assert dgemm_route(1400, 1400, 512, sms=148).kernel == TMA_128
+    assert dgemm_route(1400, 1400, 512, sms=74).kernel == WS_64
+    # one CTA per SM: 24 tiles of 128 x 64
+    assert sgemm_route(300, 500, 300, sms=148).cluster == 4
+    assert sgemm_route(300, 500, 300, sms=74).cluster == 2

@@ -50,6 +50,7 @@ struct GemmPlan {
     int tile = TILE_128x128;
     int splits = 1;  // > 1: split-K over `splits` K ranges, needs a workspace
     bool automatic = true;  // false: `splits` was asked for by the caller and is kept
+    int sm_count = 148;     // SMs planned for
 };
 
 // Workspace (in elements of T) a plan needs.

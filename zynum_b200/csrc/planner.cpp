@@ -14,6 +14,7 @@ namespace zb {
 
 GemmPlan plan_native_gemm(int m, int n, int k, int elem_bytes, int sm_count) {
     GemmPlan p;
+    p.sm_count = sm_count;
     // n == 1 or m == 1: matrix-vector kernels, K split only while the outputs
     // alone leave SMs idle.
     if (n == 1 || m == 1) {
@@ -78,7 +79,7 @@ constexpr long kMaxGridY = 65535;  // the tile kernels put column tiles on grid.
 // instead (dgemm_ws, which needs none of the plan's workspace); 0: it does not.
 int ws_cluster(int m, int n, int k, int tri, bool tma, const GemmPlan& plan) {
     if (!plan.automatic) return 0;
-    constexpr long sms = 148;
+    const long sms = plan.sm_count;
     const long t64 = (long)((m + 63) / 64) * ((n + 63) / 64);
     if (plan.tile == TILE_64x64) {
         // about one 64 x 64 tile per SM (99 .. 148 tiles on 148 SMs), which is where the plan has
@@ -107,7 +108,7 @@ int small_cluster(int m, int n, int k, const GemmPlan& plan) {
     // up to two CTAs per SM, and no fewer K ranges than the workspace route has (which splits
     // down to 64-deep slices: 256 x 256 x 1024 takes it 9.6 us, a cluster of 8 15.1)
     const long t64 = (long)((m + 63) / 64) * ((n + 63) / 64);
-    if (!plan.automatic || plan.tile != TILE_64x64 || plan.splits < 2 || 4 * t64 > 2 * 148) return 0;
+    if (!plan.automatic || plan.tile != TILE_64x64 || plan.splits < 2 || 4 * t64 > 2L * plan.sm_count) return 0;
     return k <= 256 || plan.splits == 4 ? 4 : 0;
 }
 
@@ -151,7 +152,7 @@ SgemmRoute sgemm_tile_route(int m, int n, int k, const GemmPlan& plan) {
     const int splits = std::max(1, plan.splits);
     const long t = (long)((m + 127) / 128) * ((n + 63) / 64);
     for (int c = 8; c >= 1; c /= 2)
-        if (c * t <= 148 && (c == 1 || k >= 16 * c)) {
+        if (c * t <= plan.sm_count && (c == 1 || k >= 16 * c)) {
             r.cluster = 2 * c > splits ? c : 0;
             r.halves = r.cluster && c < splits;
             break;
