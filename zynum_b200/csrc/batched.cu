@@ -670,17 +670,19 @@ ZB_DEVICE int tri_at(int r, int c) { return r >= 32 ? (kTB - 1 - r) * (kTB + 1) 
 
 // One half of the substitution as substitute_half, on the packed triangle in solve order
 // (row / column s of D is row s of a lower block, its last row minus s for an upper one, so
-// that every solve is a lower one) with its columns scaled by 1 / D[s][s]: a row's unscaled
-// final value is broadcast, so that a step is one shuffle and one FMA deep.  Lane l owns
-// solve rows l and l + 32.
+// that every solve is a lower one).  The solution value is broadcast, not the row's sum
+// against columns of D scaled by 1 / D[s][s] beforehand, which is a multiplication shallower
+// per step (5,000 solves 1.40 against 1.42 ms) but overflows where an entry's ratio to the
+// diagonal does, although the solution does not.  Lane l owns solve rows l and l + 32.
 template <int CM, int HI>
-ZB_DEVICE void substitute_tri(double (&x)[2][CM], const double* D, int sz) {
+ZB_DEVICE void substitute_tri(double (&x)[2][CM], const double* D, const double* dinv, int sz) {
     const int lane = threadIdx.x & 31;
     const int lo = 32 * HI, hi = min(sz, lo + 32);
     for (int i = lo; i < hi; ++i) {
+        const double di = dinv[i];
         double xi[CM];
 #pragma unroll
-        for (int c = 0; c < CM; ++c) xi[c] = __shfl_sync(0xffffffffu, x[HI][c], i & 31);
+        for (int c = 0; c < CM; ++c) xi[c] = __shfl_sync(0xffffffffu, x[HI][c] * di, i & 31);
         if (HI == 0) {  // every row of the second half
             const double d = D[tri_at(lane + 32, i)];
 #pragma unroll
@@ -704,8 +706,8 @@ ZB_DEVICE void substitute_packed(double (*X)[kLlXP], const double* D, const doub
     for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int c = 0; c < CM; ++c) x[h][c] = X[lane + 32 * h][warp + 8 * c];
-    substitute_tri<CM, 0>(x, D, sz);
-    if (sz > 32) substitute_tri<CM, 1>(x, D, sz);
+    substitute_tri<CM, 0>(x, D, dinv, sz);
+    if (sz > 32) substitute_tri<CM, 1>(x, D, dinv, sz);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const double s = dinv[lane + 32 * h];
@@ -875,11 +877,6 @@ trsm_batched_ll_f64(const int2* __restrict__ items, int count, int* __restrict__
                 }
             }
             __syncthreads();
-            if (!unit)  // columns of D times 1 / diagonal
-                for (int e = t; e < kLlTri; e += kThreads) {
-                    const int row = e / (kTB + 1), j = e % (kTB + 1);
-                    D[e] *= dinv[j <= kTB - 1 - row ? j : kTB - j];
-                }
             if (nch > 0)
                 for (int h = 0; h < 2; ++h) {
                     if (kh == h) {
@@ -893,8 +890,6 @@ trsm_batched_ll_f64(const int2* __restrict__ items, int count, int* __restrict__
                     }
                     __syncthreads();
                 }
-            else
-                __syncthreads();
             // the next block's first kLlAhead chunks, if none of their rows is this block's: they
             // are the first ones of a lower triangle's solved rows and the last ones of an upper's
             const int solved = upper ? n - kb - sz : kb;  // rows before this block, in solve order
