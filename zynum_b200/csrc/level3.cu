@@ -68,27 +68,29 @@ ZB_DEVICE T op_tri(const T* a, long lda, char uplo, char trans, char diag, int r
 // Block b: inverse of the diagonal block op(A)[b*64 .. , b*64 ..] of size
 // s <= 64, written column-major with ld 64 (zero outside s x s).  An upper block
 // is turned around (row and column i become 63 - i), so that every inverse is a
-// lower one.  The four 16 x 16 diagonal blocks by substitution, column j by the
-// four lanes of a quad: for each row the lanes add every fourth term of
-// sum_q L[r][q] X[q][j], two shuffles combine them, and the row's reciprocal
-// diagonal (computed once) scales the result.  Then two levels of
-// X21 = -X22 (L21 X11), 16 and 32 wide.  Bound: latency (64 serial steps of
-// substitution took 32 us for order 4096, cold; sixteen and the merges 13.6).
-constexpr int kTriT = 32;  // scratch of a merge: 32 x 33
-
+// lower one.  Column j is substituted by the four lanes of a quad, 16 rows at a
+// time: lane p adds up every fourth term of sum_q L[r][q] X[q][j], first over the
+// rows above for all sixteen sums at once, then row by row, two shuffles and the
+// row's reciprocal diagonal (computed once) each.  The dependent part of a row is
+// so one FMA, the shuffles and a product deep instead of a sum over up to 16
+// pairs of shared loads (bound: latency; the inverses of order 64 36.1 -> 17.0 us
+// a call, of order 4096 68.1 -> 32.0 with tri_inv_leaf).  Merging inverses of 16-
+// and 32-row blocks, X21 = -X22 (L21 X11), is a microsecond faster (15.8 / 30.9)
+// but not as accurate: it multiplies rounding errors by |L22| |X22|, and
+// |L X - I| came to 900 u |L| |X| on graded triangles where substitution stays
+// below 3 u.
 template <typename T>
 __host__ __device__ constexpr int tri_inv_smem() {
-    return (2 * kNB * (kNB + 1) + kTriT * (kTriT + 1) + kNB) * (int)sizeof(T);
+    return (2 * kNB * (kNB + 1) + kNB) * (int)sizeof(T);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(256) tri_inv_blocks(const T* __restrict__ a, long lda, char uplo, char trans,
                                                       char diag, int n, T* __restrict__ out) {
-    extern __shared__ __align__(16) unsigned char tri_smem[];  // 2 x 64 x 65 elements, a merge's scratch, 64 reciprocals
+    extern __shared__ __align__(16) unsigned char tri_smem[];  // 2 x 64 x 65 elements, 64 reciprocals
     T(*L)[kNB + 1] = reinterpret_cast<T(*)[kNB + 1]>(tri_smem);
     T(*X)[kNB + 1] = L + kNB;
-    T(*W)[kTriT + 1] = reinterpret_cast<T(*)[kTriT + 1]>(X + kNB);
-    T* dinv = reinterpret_cast<T*>(W + kTriT);
+    T* dinv = reinterpret_cast<T*>(X + kNB);
     grid_dependency_wait();  // may start during the tail of the kernel before it (which may write A)
     const int b0 = blockIdx.x * kNB;
     const int s = min(kNB, n - b0);
@@ -112,43 +114,32 @@ __global__ void __launch_bounds__(256) tri_inv_blocks(const T* __restrict__ a, l
     __syncthreads();
     if (t < kNB) dinv[t] = (turned(t) < s && diag != 'U') ? T(1) / L[t][t] : T(1);
     __syncthreads();
-    {
-        const int lane = t & 31, j = (t >> 5) * 8 + (lane >> 2), part = lane & 3, first = j & ~15;
-        for (int r = first; r < first + 16; ++r) {
-            T v = T(0);
-            if (r >= j)
-                for (int q = j + part; q < r; q += 4) v = fma(L[r][q], X[q][j], v);
-            v += __shfl_xor_sync(0xffffffffu, v, 1);
-            v += __shfl_xor_sync(0xffffffffu, v, 2);
-            if (r >= j && part == 0) X[r][j] = ((r == j ? T(1) : T(0)) - v) * dinv[r];
-            __syncwarp();
+    const int lane = t & 31, j = (t >> 5) * 8 + (lane >> 2), part = lane & 3;
+    for (int first = j & ~15; first < kNB; first += 16) {
+        T v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = T(0);
+        for (int q = j + part; q < first; q += 4) {
+            const T x = X[q][j];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = fma(L[first + i][q], x, v[i]);
         }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int r = first + i;
+            T w = v[i];
+            w += __shfl_xor_sync(0xffffffffu, w, 1);
+            w += __shfl_xor_sync(0xffffffffu, w, 2);
+            const T x = ((r == j ? T(1) : T(0)) - w) * dinv[r];
+            if (r >= j && part == 0) X[r][j] = x;
+            if (r >= j && ((r - j) & 3) == part) {
+#pragma unroll
+                for (int n2 = i + 1; n2 < 16; ++n2) v[n2] = fma(L[first + n2][r], x, v[n2]);
+            }
+        }
+        __syncwarp();
     }
     __syncthreads();
-    // X21 = -X22 (L21 X11) for blocks of h rows; each thread one row, `w` columns of one product
-    auto merge = [&](int h, int o, int i, int j0, int w, int wrow) {
-        T v[4];
-        for (int u = 0; u < w; ++u) v[u] = T(0);
-        for (int q = j0; q < h; ++q) {  // X11 is lower: an Inf or NaN of L21 meets no zero of it
-            const T l = L[o + h + i][o + q];
-            for (int u = 0; u < w; ++u)
-                if (q >= j0 + u) v[u] = fma(l, X[o + q][o + j0 + u], v[u]);
-        }
-        for (int u = 0; u < w; ++u) W[wrow + i][j0 + u] = v[u];
-        __syncthreads();
-        for (int u = 0; u < w; ++u) v[u] = T(0);
-        for (int q = 0; q <= i; ++q) {
-            const T l = X[o + h + i][o + h + q];
-            for (int u = 0; u < w; ++u) v[u] = fma(l, W[wrow + q][j0 + u], v[u]);
-        }
-        for (int u = 0; u < w; ++u) X[o + h + i][o + j0 + u] = T(0) - v[u];
-        __syncthreads();
-    };
-    {
-        const int pair = t >> 7, tt = t & 127;  // two pairs of 16 x 16 blocks, two columns a thread
-        merge(16, 32 * pair, tt >> 3, 2 * (tt & 7), 2, 16 * pair);
-        merge(32, 0, t >> 3, 4 * (t & 7), 4, 0);
-    }
     T* o = out + (long)blockIdx.x * kNB * kNB;
     for (int q = t; q < kNB * kNB; q += 256) {
         const int r = q % kNB, c = q / kNB;
