@@ -19,7 +19,30 @@ namespace zb {
 
 namespace {
 constexpr size_t kStagedMinBytes = size_t(2) << 20;
+
+// The driver's calls on the current context.  The caller's need not be the device's primary
+// one, which is what the runtime gives a new thread.
+struct ContextCalls {
+    CUresult(CUDAAPI* get)(CUcontext*) = nullptr;
+    CUresult(CUDAAPI* set)(CUcontext) = nullptr;
+};
+const ContextCalls& context_calls() {
+    static const ContextCalls calls = [] {
+        ContextCalls c;
+        cudaDriverEntryPointQueryResult q;
+        void *get = nullptr, *set = nullptr;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &get, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess &&
+            cudaGetDriverEntryPoint("cuCtxSetCurrent", &set, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess) {
+            c.get = reinterpret_cast<decltype(c.get)>(get);
+            c.set = reinterpret_cast<decltype(c.set)>(set);
+        }
+        return c;
+    }();
+    return calls;
 }
+}  // namespace
 
 cudaError_t PinnedSlots::reserve() {
     if (base) return cudaSuccess;
@@ -72,6 +95,10 @@ bool CopyTeam::staged(const void* host, size_t width, size_t height) {
     if (attr.type != cudaMemoryTypeUnregistered) return false;
     const int want = std::min<int>(PinnedSlots::kThreads, (int)std::thread::hardware_concurrency() / 2);
     if (want < 2 || slots_.reserve() != cudaSuccess) return false;
+    if (!context_) {
+        const ContextCalls& calls = context_calls();
+        if (!calls.set || calls.get(&context_) != CUDA_SUCCESS || !context_) return false;
+    }
     try {
         threads_.reserve(want - 1);
         while ((int)threads_.size() < want - 1) {
@@ -85,7 +112,7 @@ bool CopyTeam::staged(const void* host, size_t width, size_t height) {
 }
 
 void CopyTeam::loop(int id, long seen) {
-    cudaSetDevice(device_);
+    const bool bound = context_calls().set(context_) == CUDA_SUCCESS;  // if not, the others do its share
     for (;;) {
         // the transfers of one call follow each other within microseconds: poll for the next
         // one for a while before sleeping (a wake-up costs 50 to 100 us here)
@@ -98,7 +125,7 @@ void CopyTeam::loop(int id, long seen) {
             if (quit_) return;
             seen = generation_;
         }
-        work(id);
+        if (bound) work(id);
         std::lock_guard<std::mutex> lock(mu_);
         if (--busy_ == 0) finish_.notify_one();
     }

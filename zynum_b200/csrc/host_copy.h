@@ -8,6 +8,7 @@
 #include <thread>
 #include <vector>
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 namespace zb {
@@ -24,11 +25,11 @@ struct PinnedSlots {
 };
 
 // The copying threads of one host call: started on the first transfer that takes
-// them, joined by the destructor.  The caller holds the context's mutex, so one
-// team uses the slots at a time.
+// them, in the calling thread's CUDA context, joined by the destructor.  The caller
+// holds the context's mutex, so one team uses the slots at a time.
 class CopyTeam {
   public:
-    CopyTeam(PinnedSlots& slots, int device) : slots_(slots), device_(device) {}
+    explicit CopyTeam(PinnedSlots& slots) : slots_(slots) {}
     ~CopyTeam();
     CopyTeam(const CopyTeam&) = delete;
     CopyTeam& operator=(const CopyTeam&) = delete;
@@ -57,7 +58,7 @@ class CopyTeam {
     void loop(int id, long seen);
 
     PinnedSlots& slots_;
-    int device_;
+    CUcontext context_ = nullptr;  // the calling thread's, for the copying threads
     std::vector<std::thread> threads_;
     std::mutex mu_;
     std::condition_variable start_, finish_;
