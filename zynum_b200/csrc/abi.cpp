@@ -215,7 +215,8 @@ void host_gemm_panels(const char* routine, Context& cx, int panels, char ta, cha
     };
     for (auto& x : ev)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&x, cudaEventDisableTiming);
-    CopyTeam team(cx.slots);
+    CopyTeam team(cx.slots, {{a, (size_t)ra * ca * es}, {b, (size_t)k * n * es},
+                             {c, beta == T(0) ? 0 : (size_t)m * n * es}, {c, (size_t)m * n * es}});
     // FP64 through the CRT Ozaki scheme: one plan for the full panel width,
     // op(A)'s residues computed by the first panel and reused by the others (its row
     // scaling depends on op(A) alone, each column of op(B) is scaled independently, so
@@ -325,7 +326,8 @@ void host_gemm(const char* routine, char ta, char tb, int m, int n, int k, T alp
         host_gemm_panels<T>(routine, cx, panels, ta, tb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, da, db, dc);
         return;
     }
-    CopyTeam team(cx.slots);
+    CopyTeam team(cx.slots, {{a, quick ? 0 : (size_t)ra * ca * es}, {b, quick ? 0 : (size_t)rb * cb * es},
+                             {c, beta == T(0) ? 0 : (size_t)m * n * es}, {c, (size_t)m * n * es}});
     if (!quick) {
         e = team.upload(da, (size_t)ra * es, a, (size_t)lda * es, (size_t)ra * es, ca, st);
         if (e == cudaSuccess) e = team.upload(db, (size_t)rb * es, b, (size_t)ldb * es, (size_t)rb * es, cb, st);
@@ -471,7 +473,8 @@ void host_complex_gemm(const char* routine, char ta, char tb, int m, int n, int 
     T* da = static_cast<T*>(cx.stage_a.ptr);
     T* db = static_cast<T*>(cx.stage_b.ptr);
     T* dc = static_cast<T*>(cx.stage_c.ptr);
-    CopyTeam team(cx.slots);
+    CopyTeam team(cx.slots, {{a, quick ? 0 : (size_t)ra * ca * es}, {b, quick ? 0 : (size_t)rb * cb * es},
+                             {c, beta0 ? 0 : (size_t)m * n * es}, {c, (size_t)m * n * es}});
     if (!quick) {
         e = team.upload(da, (size_t)ra * es, a, (size_t)lda * es, (size_t)ra * es, ca, st);
         if (e == cudaSuccess) e = team.upload(db, (size_t)rb * es, b, (size_t)ldb * es, (size_t)rb * es, cb, st);

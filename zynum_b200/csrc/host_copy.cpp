@@ -6,8 +6,8 @@
 // eight host threads copy 512 KB chunks into pinned slots and enqueue each
 // chunk's device copy themselves; with two slots a thread fills one while the
 // other is on the link.  dgemm_ 2048^3 8.1 -> 4.0 ms a call, 1024^3 2.2 -> 1.4.
-// Page-locked memory and transfers under 2 MB (starting the threads would not
-// pay) keep cudaMemcpy2DAsync.
+// Page-locked memory keeps cudaMemcpy2DAsync, and so do transfers under 2 MB and
+// a call's only larger one up to 8 MB: starting the threads would not pay.
 #include "host_copy.h"
 
 #include <algorithm>
@@ -18,7 +18,20 @@
 namespace zb {
 
 namespace {
+// Threads are started per call.  Two transfers of 2 MB repay it (dgemm_ 512^3, three: 460 ->
+// 420 us; C of 520 x 520 up and down: 500 -> 340), one does from about 8 MB (one upload of 4 MB
+// 335 -> 395 us, of 11 MB 690 -> 650; one download of 2 MB 208 -> 245, of 8 MB 560 -> 530).
 constexpr size_t kStagedMinBytes = size_t(2) << 20;
+constexpr size_t kLoneMinBytes = size_t(8) << 20;
+
+bool pageable(const void* host) {
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return attr.type == cudaMemoryTypeUnregistered;
+}
 
 // The driver's calls on the current context.  The caller's need not be the device's primary
 // one, which is what the runtime gives a new thread.
@@ -74,6 +87,12 @@ void PinnedSlots::release() {
     base = nullptr;
 }
 
+CopyTeam::CopyTeam(PinnedSlots& slots, std::initializer_list<Transfer> transfers) : slots_(slots) {
+    int large = 0;
+    for (const Transfer& t : transfers) large += t.bytes >= kStagedMinBytes && pageable(t.host);
+    min_bytes_ = large > 1 ? kStagedMinBytes : kLoneMinBytes;
+}
+
 CopyTeam::~CopyTeam() {
     {
         std::lock_guard<std::mutex> lock(mu_);
@@ -86,14 +105,10 @@ CopyTeam::~CopyTeam() {
 
 // Whether this transfer goes through the slots; starts the threads the first time.
 bool CopyTeam::staged(const void* host, size_t width, size_t height) {
-    if (width * height < kStagedMinBytes) return false;
-    cudaPointerAttributes attr;
-    if (cudaPointerGetAttributes(&attr, host) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    if (attr.type != cudaMemoryTypeUnregistered) return false;
-    const int want = std::min<int>(PinnedSlots::kThreads, (int)std::thread::hardware_concurrency() / 2);
+    const size_t bytes = width * height, slot = PinnedSlots::kSlotBytes;
+    if (bytes < min_bytes_ || !pageable(host)) return false;
+    int want = std::min<int>(PinnedSlots::kThreads, (int)std::thread::hardware_concurrency() / 2);
+    want = (int)std::min<size_t>(want, (bytes + slot - 1) / slot);  // no more than there are chunks
     if (want < 2 || slots_.reserve() != cudaSuccess) return false;
     if (!context_) {
         const ContextCalls& calls = context_calls();

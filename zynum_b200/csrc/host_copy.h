@@ -4,6 +4,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstddef>
+#include <initializer_list>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -29,7 +30,12 @@ struct PinnedSlots {
 // holds the context's mutex, so one team uses the slots at a time.
 class CopyTeam {
   public:
-    explicit CopyTeam(PinnedSlots& slots) : slots_(slots) {}
+    struct Transfer {
+        const void* host;
+        size_t bytes;
+    };
+    // transfers: what the call will copy, for the decision whether threads pay.
+    CopyTeam(PinnedSlots& slots, std::initializer_list<Transfer> transfers);
     ~CopyTeam();
     CopyTeam(const CopyTeam&) = delete;
     CopyTeam& operator=(const CopyTeam&) = delete;
@@ -58,6 +64,7 @@ class CopyTeam {
     void loop(int id, long seen);
 
     PinnedSlots& slots_;
+    size_t min_bytes_;             // smallest transfer that takes the threads
     CUcontext context_ = nullptr;  // the calling thread's, for the copying threads
     std::vector<std::thread> threads_;
     std::mutex mu_;
