@@ -551,49 +551,7 @@ trsm_batched_kernel(const int2* __restrict__ items, int count, int* __restrict__
                     cp_async_wait<0>();
                 }
                 __syncthreads();
-                if constexpr (sizeof(T) == 8) {
-                    // FP64: the chunk update B[c0 .. c0 + rows) -= P^T X as 16 x 8 DMMA tiles;
-                    // warp w takes row tile w % 4 and column tiles 4 (w / 4) .. +3 (those below r)
-                    const int g = lane >> 2, tq = lane & 3, rt = warp & 3, ct0 = (warp >> 2) * 4;
-                    const int nct = (r + 7) / 8;
-                    double acc[4][4] = {}, bv[4][4];
-                    if (ct0 < nct) {
-                        // the B values this warp updates, in flight before the products
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-#pragma unroll
-                            for (int v = 0; v < 4; ++v) {
-                                const int row = 16 * rt + g + 8 * (v >> 1), col = 8 * (ct0 + u) + 2 * tq + (v & 1);
-                                bv[u][v] = (ct0 + u < nct && row < rows && col < r) ? B[c0 + row + (long)col * lb]
-                                                                                   : 0.0;
-                            }
-                        for (int k8 = 0; k8 < (sz + 7) / 8; ++k8) {
-                            double af[4];
-#pragma unroll
-                            for (int v1 = 0; v1 < 2; ++v1)
-#pragma unroll
-                                for (int v0 = 0; v0 < 2; ++v0)
-                                    af[v0 + 2 * v1] = P[8 * k8 + tq + 4 * v1][16 * rt + g + 8 * v0];
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) {
-                                if (ct0 + u >= nct) break;
-                                double bf[2];
-#pragma unroll
-                                for (int v = 0; v < 2; ++v) bf[v] = X[8 * k8 + tq + 4 * v][8 * (ct0 + u) + g];
-                                dmma_16x8x8(acc[u], af, bf);
-                            }
-                        }
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            if (ct0 + u >= nct) break;
-#pragma unroll
-                            for (int v = 0; v < 4; ++v) {
-                                const int row = 16 * rt + g + 8 * (v >> 1), col = 8 * (ct0 + u) + 2 * tq + (v & 1);
-                                if (row < rows && col < r) B[c0 + row + (long)col * lb] = bv[u][v] - acc[u][v];
-                            }
-                        }
-                    }
-                } else if (4 * cg < r) {
+                if (4 * cg < r) {
                     // the B values this thread updates, fetched before the K loop
                     T bv[4][4];
 #pragma unroll

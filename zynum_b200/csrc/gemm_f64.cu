@@ -326,10 +326,7 @@ dgemm_cluster_kernel(int M, int N, int K, int k_chunk, double alpha, const doubl
 #pragma unroll
             for (int v = 0; v < 4; ++v)
                 P[(wn + j * 8 + 2 * t + (v & 1)) * kCPitch + wm + i * 16 + g + 8 * (v >> 1)] = acc[i][j][v];
-    if (splits > 1)
-        cluster_sync();
-    else
-        __syncthreads();
+    cluster_sync();
     // CTA `rank` sums, in rank order, and writes columns rank * 64 / splits ..
     const int cols = kCN / splits, c_first = rank * cols;
     for (int q = threadIdx.x; q < cols * (kCM / 2); q += kCThreads) {
@@ -338,16 +335,11 @@ dgemm_cluster_kernel(int M, int N, int K, int k_chunk, double alpha, const doubl
         if (row >= M || col >= N) continue;
         const uint32_t at = smem_u32(P + c * kCPitch + r);
         double x0 = 0.0, x1 = 0.0;
-        if (splits == 1) {
-            x0 = P[c * kCPitch + r];
-            x1 = P[c * kCPitch + r + 1];
-        } else {
-            for (int z = 0; z < splits; ++z) {
-                double y0, y1;
-                ld_cluster_f64x2(mapa_shared(at, z), y0, y1);
-                x0 += y0;
-                x1 += y1;
-            }
+        for (int z = 0; z < splits; ++z) {
+            double y0, y1;
+            ld_cluster_f64x2(mapa_shared(at, z), y0, y1);
+            x0 += y0;
+            x1 += y1;
         }
         double* cp = C + (long)col * ldc + row;
         const bool in0 = tri == 0 || (tri == 1 ? row <= col : row >= col);
@@ -362,7 +354,7 @@ dgemm_cluster_kernel(int M, int N, int K, int k_chunk, double alpha, const doubl
         if (in0) cp[0] = x0;
         if (in1) cp[1] = x1;
     }
-    if (splits > 1) cluster_sync();  // no CTA leaves while its partial tile may be read
+    cluster_sync();  // no CTA leaves while its partial tile may be read
 }
 
 __global__ void dgemm_splitk_reduce(int M, int N, int splits, const double* __restrict__ W, double alpha, double beta,

@@ -55,7 +55,7 @@ constexpr int kFGroups = 4, kFGroupWarps = 4;                  // FP32, one stag
 constexpr int kStagesAll = kGroups * kGroupStages;
 constexpr int kKThreads = kGroups * kGroupWarps * 32;
 static_assert(kKThreads == kFGroups * kFGroupWarps * 32, "both kernels run the same block");
-constexpr int kKBM = 16;                                    // FP64 rows per block
+constexpr int kKBM = 16;                                    // FP64 rows per block (one 128-byte box)
 constexpr int kKABytes = kKBM * kKK * 8;                    // 8 KB per stage
 constexpr int kKBBytes = kKN * kKK * 8;                     // 32 KB, resident
 constexpr size_t kKSmem = 1024 + (size_t)kStagesAll * kKABytes + kKBBytes + 256;
@@ -132,10 +132,9 @@ dgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     const WaitCtl W{abort_flag, nullptr, P.report, P.wait_ns};
     uint8_t* const stage0 = smem + grp * kGroupStages * kKABytes;
     auto boxes = [&](uint32_t st, uint64_t* bar, int i0) {
-        if (A_MN) {  // 2 boxes of 64 k-rows x 16 m
-#pragma unroll
-            for (int b = 0; b < kKBM / 16; ++b) tma_load_2d(st + b * 8192, &tmA, bar, i0 + 16 * b, 0);
-        } else {  // 4 boxes of 32 m-rows x 16 k
+        if (A_MN) {  // one box of 64 k-rows x 16 m
+            tma_load_2d(st, &tmA, bar, i0, 0);
+        } else {  // 4 boxes of 16 m-rows x 16 k
 #pragma unroll
             for (int b = 0; b < kKK / 16; ++b) tma_load_2d(st + b * (kKBM * 128), &tmA, bar, 16 * b, i0);
         }
@@ -169,13 +168,13 @@ dgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     }
     __syncthreads();
 
-    const int wm = 0, wn = wq * 32;
+    const int wn = wq * 32;
     const int g = lane >> 2, t = lane & 3;
     const int ks8 = (P.K + 7) / 8;
     const int nfrag = max(0, min(4, (P.N - wn + 7) / 8));  // 8-column fragments inside op(B)
     uint32_t a_off[2], b_off[4];
 #pragma unroll
-    for (int v = 0; v < 2; ++v) a_off[v] = A_MN ? mn_off(wm + 2 * g, 2 * t + v) : k_off<kKBM>(wm + 2 * g + v, 2 * t);
+    for (int v = 0; v < 2; ++v) a_off[v] = A_MN ? mn_off(2 * g, 2 * t + v) : k_off<kKBM>(2 * g + v, 2 * t);
 #pragma unroll
     for (int j = 0; j < 4; ++j) b_off[j] = k_off<kKN>(wn + 8 * j + ((g >> 1) | ((g & 1) << 2)), 2 * t);
 
@@ -186,7 +185,7 @@ dgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         const int q = n & (kGroupStages - 1);
         const uint32_t ph = (uint32_t)(n / kGroupStages) & 1u;
         const uint8_t* sa = stage0 + q * kKABytes;
-        const int row = blk * kKBM + wm + 2 * g;
+        const int row = blk * kKBM + 2 * g;
         // beta * C loads first: their latency overlaps this block's products
         double cin[4][2][2];
 #pragma unroll
@@ -240,7 +239,7 @@ dgemm_skinny_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
                     if (j < nfrag) dmma_16x8x8(acc[j], af, bf[j]);
             }
         }
-        // the group's four warps are done with the stage (or leave together)
+        // the group's warps are done with the stage (or leave together)
         if (!(ok = group_bar_and<kGroupWarps>(grp, ok))) break;
         if (wq == 0 && lane == 0)
             feed_stage(&full[grp * kGroupStages + q], smem_u32(sa), kKABytes, blk + kGroupStages * step, kKBM,
