@@ -78,12 +78,32 @@ def test_cluster_routes_need_no_workspace():
 
 def test_rules_follow_the_sm_count():
     """The routing rules use the SM count that the plan was made for (a partitioned GPU has fewer)."""
-    # up to two CTAs per SM: 49 tiles in clusters of four are 196 CTAs
-    assert dgemm_route(400, 400, 200, sms=148).kernel == CLUSTER_64
-    assert dgemm_route(400, 400, 200, sms=74).kernel == TILES
+    # up to two CTAs per SM: 56 tiles in clusters of four are 224 CTAs
+    assert dgemm_route(448, 512, 200, sms=148).kernel == CLUSTER_64
+    assert dgemm_route(448, 512, 200, sms=74).kernel == TILES
     # rounds of tiles: 121 tiles of 128 x 128 are one round on 148 SMs, two on 74 (484 of 64 x 64: seven)
     assert dgemm_route(1400, 1400, 512, sms=148).kernel == TMA_128
     assert dgemm_route(1400, 1400, 512, sms=74).kernel == WS_64
     # one CTA per SM: 24 tiles of 128 x 64
     assert sgemm_route(300, 500, 300, sms=148).cluster == 4
     assert sgemm_route(300, 500, 300, sms=74).cluster == 2
+
+
+@pytest.mark.parametrize("m,n,k,kernel", [
+    (256, 256, 256, CLUSTER_64), (128, 1024, 300, CLUSTER_64),       # up to 33 tiles: an SM for each CTA
+    (384, 384, 160, CLUSTER_64), (384, 384, 256, TILES),             # 36 tiles: 144 CTAs of the plan fit, clusters do not
+    (448, 448, 192, TILES), (448, 448, 256, CLUSTER_64), (448, 448, 300, TILES),  # 49 tiles, three and four ranges
+    (512, 512, 512, CLUSTER_64), (512, 512, 768, CLUSTER_64), (512, 512, 1024, TILES),
+    (448, 640, 512, CLUSTER_64), (520, 500, 512, TILES), (520, 500, 128, TILES),  # 70 and 72 tiles
+])
+def test_small_dgemm_clusters(m, n, k, kernel):
+    assert dgemm_route(m, n, k, tma=False).kernel == kernel
+
+
+@pytest.mark.parametrize("m,n,k,cluster", [
+    (128, 960, 4000, 8), (128, 1024, 1500, 8), (128, 1152, 2048, 0), (160, 558, 3017, 0),  # 15, 16, 18 tiles
+    (128, 2112, 1500, 4), (128, 2304, 511, 4), (128, 2304, 1500, 0), (128, 2368, 4000, 0),  # 33, 36, 37 tiles
+    (1024, 576, 4000, 2),  # 72 tiles
+])
+def test_sgemm_clusters_that_share_sms(m, n, k, cluster):
+    assert sgemm_route(m, n, k).cluster == cluster

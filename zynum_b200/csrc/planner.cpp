@@ -102,14 +102,32 @@ int ws_cluster(int m, int n, int k, int tri, bool tma, const GemmPlan& plan) {
     return r64 < 0.98 * r128 && tma ? 1 : 0;
 }
 
+// CTAs of `c`-clusters that run with an SM each.  A cluster lives inside one GPC, so up to
+// c - 1 SMs of every GPC stay free: on 148 SMs 15 clusters of eight run side by side, 33 of
+// four and 74 of two; the 16th, 34th, ... share SMs with the others, and their launch takes
+// twice as long as the SM count suggests.
+long cluster_ctas(int c, long sms) { return c > 2 ? sms - 7 * c / 2 : sms; }
+
 // Cluster size with which a planned small product runs on the 64 x 64 cluster tiles
 // (dgemm_cluster_kernel: one launch, none of the plan's workspace); 0: it does not.
+// Never fewer K ranges than the plan, which splits down to 64-deep slices (256 x 256 x 1024 in
+// 16 ranges 9.6 us, a cluster of 8 15.1).  Microseconds on the device, plan / cluster of four.
 int small_cluster(int m, int n, int k, const GemmPlan& plan) {
-    // up to two CTAs per SM, and no fewer K ranges than the workspace route has (which splits
-    // down to 64-deep slices: 256 x 256 x 1024 takes it 9.6 us, a cluster of 8 15.1)
-    const long t64 = (long)((m + 63) / 64) * ((n + 63) / 64);
-    if (!plan.automatic || plan.tile != TILE_64x64 || plan.splits < 2 || 4 * t64 > 2L * plan.sm_count) return 0;
-    return k <= 256 || plan.splits == 4 ? 4 : 0;
+    const long t64 = (long)((m + 63) / 64) * ((n + 63) / 64), sms = plan.sm_count;
+    if (!plan.automatic || plan.tile != TILE_64x64 || plan.splits < 2) return 0;
+    if (k > 256 && plan.splits != 4) return 0;
+    // an SM for each CTA (up to 33 tiles): saves the second launch (33 tiles, k = 192: 8.5 / 6.7;
+    // 16 tiles, k = 256: 6.6 / 6.8, and 11.4 / 9.3 a call)
+    if (4 * t64 <= cluster_ctas(4, sms)) return 4;
+    // more than two CTAs for an SM: the last clusters run alone (72 tiles, k = 512: 0.75 x)
+    if (4 * t64 > sms + cluster_ctas(4, sms)) return 0;
+    // two CTAs on an SM: where the plan's ranges are twice as long (k = 160: 1.05 - 1.2 x) or
+    // share SMs too (50 tiles, k = 192: 1.26 x; 34 - 37 tiles, k = 192 .. 319, where they have an
+    // SM each: 0.78 - 0.99 x; 40 - 59 tiles with four ranges, k = 257 .. 319: 0.77 - 1.04 x)
+    if (k <= 256) return plan.splits == 2 || plan.splits * t64 > sms ? 4 : 0;
+    // 60 to 70 tiles, which the plan gives four ranges whatever K: 1.02 - 1.08 x up to k = 768,
+    // 0.95 - 1.01 x at 1024
+    return 2 * sms / t64 == 4 && k <= 768 ? 4 : 0;
 }
 
 }  // namespace
@@ -146,14 +164,18 @@ DgemmRoute dgemm_tile_route(int m, int n, int k, int tri, bool tma, const GemmPl
 // The largest cluster with at most one CTA per SM and 16-deep ranges, where its CTAs then have
 // less to do than the plan's: (K / c) x 64 columns against (K / splits) x 128 (1024^3: c = 1
 // against two K ranges, 65 against 61 us, keeps the plan; 300 x 300 x 4000, c = 8 against 15:
-// 36.9 / 37.1; 256 x 256 x 262144, c = 8 against 37, keeps it).
+// 36.9 / 37.1; 256 x 256 x 262144, c = 8 against 37, keeps it).  Clusters that share SMs have
+// half the rate: they need shorter ranges than the plan's (18 tiles, c = 8: k = 1500, five
+// ranges, 1.5 x; 2048, eight, 0.97; 4000, fifteen, 0.64.  36 tiles, c = 4: k = 511 2.9 x, 1500,
+// five ranges, 0.91).
 SgemmRoute sgemm_tile_route(int m, int n, int k, const GemmPlan& plan) {
     SgemmRoute r;
     const int splits = std::max(1, plan.splits);
     const long t = (long)((m + 127) / 128) * ((n + 63) / 64);
     for (int c = 8; c >= 1; c /= 2)
         if (c * t <= plan.sm_count && (c == 1 || k >= 16 * c)) {
-            r.cluster = 2 * c > splits ? c : 0;
+            const bool alone = c * t <= cluster_ctas(c, plan.sm_count);
+            r.cluster = (alone ? 2 * c : c) > splits ? c : 0;
             r.halves = r.cluster && c < splits;
             break;
         }
