@@ -611,6 +611,9 @@ trsm_batched_kernel(const int2* __restrict__ items, int count, int* __restrict__
 // right-hand sides) 1.81 -> 1.42 ms, 1,800 of them 1.40 -> 0.97; with two 32-deep stages
 // and whole problems on two CTAs before.  A fourth stage is slower (1.58 ms: it leaves L1 too
 // little), two stages or no chunk ahead 1.48 / 1.42 (the latter 3 % slower on small batches).
+// An item's successor is claimed with its last block: claimed at its start, the last items of a
+// batch waited behind others while CTAs were idle (148 equal problems ran on 56 SMs; 500 of
+// order 256 with 32 right-hand sides 216 -> 156 us, 148 of them 115 -> 61).
 constexpr int kLlK = 16;                               // K chunk
 constexpr int kLlStages = 3;
 constexpr int kLlPA = kTB + 4;                         // op(A) chunk [k][row]
@@ -690,7 +693,6 @@ trsm_batched_ll_f64(const int2* __restrict__ items, int count, int* __restrict__
     __shared__ int claim_slot[2];
     Claim cl{next, claim_slot};
     for (int w = cl.first(); w < count; w = cl.advance()) {
-        cl.prefetch();
         const int2 item = items[w];
         const int q = item.x, n = dims[2 * q], r = min(kTrsmCols, dims[2 * q + 1] - item.y);
         const double* A = a[q];
@@ -736,6 +738,7 @@ trsm_batched_ll_f64(const int2* __restrict__ items, int count, int* __restrict__
         };
         int ahead = 0;  // chunks of this block already loading
         for (int s = 0; s < nblk; ++s) {
+            if (s + 1 == nblk) cl.prefetch();  // late: a claimed item waits for the end of this one
             const int kb = (upper ? nblk - 1 - s : s) * kTB, sz = min(kTB, n - kb);
             const int nch = ((upper ? n - kb - sz : kb) + kLlK - 1) / kLlK;
             // diagonal block in solve order, packed: element (sr, sc), sc <= sr, at base + sr dr + sc dc;
@@ -937,7 +940,7 @@ cudaError_t launch_trsm_batched(const int2* items, int count, int* next, const i
     if ((e = cudaMemsetAsync(next, 0, sizeof(int), st)) != cudaSuccess) return e;
     prof_begin(st);
     if (dtype == BATCH_F64)
-        trsm_batched_ll_f64<<<grid, kThreads, sm_ll, st>>>(
+        trsm_batched_ll_f64<<<std::min(grid, count), kThreads, sm_ll, st>>>(
             items, count, next, dims, uplo, trans, diag, *static_cast<const double*>(alpha),
             reinterpret_cast<const double* const*>(a), lda, reinterpret_cast<double* const*>(b), ldb);
     else
