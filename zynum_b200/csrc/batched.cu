@@ -613,7 +613,9 @@ trsm_batched_kernel(const int2* __restrict__ items, int count, int* __restrict__
 // little), two stages or no chunk ahead 1.48 / 1.42 (the latter 3 % slower on small batches).
 // An item's successor is claimed with its last block: claimed at its start, the last items of a
 // batch waited behind others while CTAs were idle (148 equal problems ran on 56 SMs; 500 of
-// order 256 with 32 right-hand sides 216 -> 156 us, 148 of them 115 -> 61).
+// order 256 with 32 right-hand sides 216 -> 156 us, 148 of them 115 -> 61).  X is formed from
+// the DMMA registers of one half; a pass of its own took 5,200 clocks a block, with bank
+// conflicts of four and eight at a pitch of 36 (those 500: 156 -> 139 us).
 constexpr int kLlK = 16;                               // K chunk
 constexpr int kLlStages = 3;
 constexpr int kLlPA = kTB + 4;                         // op(A) chunk [k][row]
@@ -621,7 +623,7 @@ constexpr int kLlPX = kLlK + 4;                        // X chunk [column][k]: c
 constexpr int kLlStage = kLlK * kLlPA + kTrsmCols * kLlPX;
 constexpr int kLlRing = kLlStages * kLlStage;
 constexpr int kLlAhead = 1;                            // chunks of the next block loaded before the substitution
-constexpr int kLlXP = kTrsmCols + 4;
+constexpr int kLlXP = kTrsmCols + 1;                   // a lane per row reads a column without bank conflicts
 constexpr int kLlTri = 32 * (kTB + 1);                 // packed triangle of the diagonal block
 static_assert(kTB * kLlXP <= (kLlStages - kLlAhead) * kLlStage, "the solve block reuses the last stages");
 
@@ -822,35 +824,36 @@ trsm_batched_ll_f64(const int2* __restrict__ items, int count, int* __restrict__
             }
             cp_async_wait<0>();
             __syncthreads();
-            // the block to solve, in solve order: X = alpha B_block, then minus both halves' sums
+            // the block to solve, in solve order: X = alpha B_block minus one half's sums, then the
+            // other's (columns past r are not used)
             if (t < kTB) dinv[t] = (unit || t >= sz) ? 1.0 : 1.0 / D[tri_at(t, t)];
-            {
-                double bv[kTB * kTrsmCols / kThreads];
 #pragma unroll
-                for (int u = 0; u < kTB * kTrsmCols / kThreads; ++u) {
-                    const int e = u * kThreads + t, rr = e % kTB, cc = e / kTB;
-                    bv[u] = (rr < sz && cc < r) ? B[kb + (upper ? sz - 1 - rr : rr) + (long)cc * lb] : 0.0;
-                }
-#pragma unroll
-                for (int u = 0; u < kTB * kTrsmCols / kThreads; ++u) {
-                    const int e = u * kThreads + t;
-                    X[e % kTB][e / kTB] = alpha * bv[u];
-                }
-            }
-            __syncthreads();
-            if (nch > 0)
-                for (int h = 0; h < 2; ++h) {
-                    if (kh == h) {
+            for (int h = 0; h < 2; ++h) {
+                if (kh == h && (h == 0 || nch > 0)) {
+                    double bv[4][4];
+                    if (h == 0) {
 #pragma unroll
                         for (int u = 0; u < 4; ++u)
 #pragma unroll
                             for (int v = 0; v < 4; ++v) {
                                 const int row = 16 * rt + g + 8 * (v >> 1), col = 8 * u + 2 * tq + (v & 1);
-                                if (u < nct && col < r && row < sz) X[upper ? sz - 1 - row : row][col] -= acc[u][v];
+                                bv[u][v] = (row < sz && col < r) ? B[kb + row + (long)col * lb] : 0.0;
                             }
                     }
-                    __syncthreads();
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+#pragma unroll
+                        for (int v = 0; v < 4; ++v) {
+                            const int row = 16 * rt + g + 8 * (v >> 1), col = 8 * u + 2 * tq + (v & 1);
+                            double* x = &X[upper && row < sz ? sz - 1 - row : row][col];
+                            if (h == 0)
+                                *x = __dmul_rn(alpha, bv[u][v]) - acc[u][v];  // alpha B rounded, as BLAS scales it first
+                            else if (row < sz)
+                                *x -= acc[u][v];
+                        }
                 }
+                __syncthreads();
+            }
             // the next block's first kLlAhead chunks, if none of their rows is this block's: they
             // are the first ones of a lower triangle's solved rows and the last ones of an upper's
             const int solved = upper ? n - kb - sz : kb;  // rows before this block, in solve order
