@@ -41,6 +41,7 @@ def test_routes(blas, oracle, ta, tb, shape, route, beta):
     (1000, 1500, (TMA_128, 2, 1)),
     (900, 1025, (TMA_128, 2, 1)),
     (1200, 1300, (WS_64, 1, 1)),
+    (2200, 260, (WS_64, 1, 1)),
     (576, 1000, (TILES, 1, 3)),
 ])
 def test_triangle_routes(blas, uplo, trans, n, k, route):

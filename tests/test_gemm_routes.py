@@ -107,3 +107,9 @@ def test_small_dgemm_clusters(m, n, k, kernel):
 ])
 def test_sgemm_clusters_that_share_sms(m, n, k, cluster):
     assert sgemm_route(m, n, k).cluster == cluster
+
+
+@pytest.mark.parametrize("n,kernel", [(1300, WS_64), (1500, WS_64), (1700, TMA_128), (2048, TMA_128), (2200, WS_64),
+                                      (2400, WS_64), (2700, TMA_128), (2876, TMA_128), (2950, WS_64), (3600, TMA_128)])
+def test_triangle_tiles(n, kernel):
+    assert dgemm_route(n, n, 1335, tri=1).kernel == kernel

@@ -98,7 +98,12 @@ int ws_cluster(int m, int n, int k, int tri, bool tma, const GemmPlan& plan) {
     // 1689 / 1628, 1536^3, one round of 128 x 128 tiles, 212 / 229)
     const long m1 = (m + 127) / 128, n1 = (n + 127) / 128, m6 = (m + 63) / 64;
     const long live1 = tri ? m1 * (m1 + 1) / 2 : m1 * n1, live6 = tri ? m6 * (m6 + 1) / 2 : t64;
-    const double r128 = 4.0 * ((live1 + sms - 1) / sms) / 0.955, r64 = ((live6 + sms - 1) / sms) / 0.90;
+    const double r128 = 4.0 * ((live1 + sms - 1) / sms) / 0.955;
+    double r64 = ((live6 + sms - 1) / sms) / 0.90;
+    // a triangle's CTAs without a tile leave at once, and the others land unevenly: 0.6 to 1.4
+    // tiles over the average load of an SM, and never under 3.2 (order 2876, k 1335: 377 us on
+    // 128 x 128 tiles, 413 on these; order 2200: 376 / 267; order 1700, lower: 193 / 206)
+    if (tri) r64 = std::max((double)live6 / sms + 1.2, 3.2) / 0.90;
     return r64 < 0.98 * r128 && tma ? 1 : 0;
 }
 
