@@ -603,19 +603,20 @@ trsm_batched_kernel(const int2* __restrict__ items, int count, int* __restrict__
 // written back to B once.  The diagonal block's copy is in flight during the products, the
 // next block's first chunk during the substitution.
 //
-// Bound: latency, per 64-row block about 3 us to issue the copies, 0.8 us per chunk, 4 to
-// form X and 6.5 for the substitution; op(A) once through HBM is a quarter of the time.  So
-// the split is for more independent blocks per SM and shorter chains: items of 32 columns
-// (a problem with 64 is two items and its chain half as long), the triangle packed into
-// 16.6 KB and a ring of 41 KB for three CTAs per SM.  5,000 problems (n 16..1024, 1..64
-// right-hand sides) 1.81 -> 1.42 ms, 1,800 of them 1.40 -> 0.97; with two 32-deep stages
-// and whole problems on two CTAs before.  A fourth stage is slower (1.58 ms: it leaves L1 too
+// Bound: latency.  Clocks per 64-row block with one item on an SM, 1 / 32 right-hand sides: 3,000
+// to issue the diagonal block's copies, 600 / 1,000 a chunk, 1,800 / 2,200 to form X, 1,000 to
+// issue the next block's first chunk, 5,600 / 9,500 for the substitution, 170 / 1,100 to write; op(A)
+// once through HBM is a third of the time of 5,000 problems (n 16..1024, 1..64 right-hand sides).
+// So the split is for more independent blocks per SM and shorter chains: items of 32 columns (a
+// problem with 64 is two items and its chain half as long), the triangle packed into 16.6 KB and
+// a ring of 41 KB for three CTAs per SM.  Those 5,000 problems 1.81 -> 1.42 ms, against whole
+// problems in two 32-deep stages on two CTAs; a fourth stage is slower (1.58 ms: it leaves L1 too
 // little), two stages or no chunk ahead 1.48 / 1.42 (the latter 3 % slower on small batches).
 // An item's successor is claimed with its last block: claimed at its start, the last items of a
 // batch waited behind others while CTAs were idle (148 equal problems ran on 56 SMs; 500 of
-// order 256 with 32 right-hand sides 216 -> 156 us, 148 of them 115 -> 61).  X is formed from
-// the DMMA registers of one half; a pass of its own took 5,200 clocks a block, with bank
-// conflicts of four and eight at a pitch of 36 (those 500: 156 -> 139 us).
+// order 256 with 32 right-hand sides 216 -> 156 us, 148 of them 115 -> 61; the 5,000 1.42 ->
+// 1.32 ms).  X is formed from the DMMA registers of one half; a pass of its own took 5,200 clocks
+// a block, with bank conflicts of four and eight at a pitch of 36 (156 -> 139 us; 1.32 -> 1.24 ms).
 constexpr int kLlK = 16;                               // K chunk
 constexpr int kLlStages = 3;
 constexpr int kLlPA = kTB + 4;                         // op(A) chunk [k][row]

@@ -12,10 +12,10 @@
 // 4-column halves so that every shared load is a conflict-free float4.  Two
 // rows of a column share one fma.rn.f32x2 (each half rounded as fmaf, so the
 // result is the same bit for bit): scalar FFMA was issue-bound at 85 % of the
-// slots, packed it takes half of them and the register file's operand reads
-// bound it (a register-only loop of this tile reaches 59.5 TFLOP/s packed, with
-// op(B)'s element duplicated by moves as here, and 49 scalar).  4096^3: 2654 ->
-// 2543 us (54.0 TFLOP/s), 8192^3 NT 53.7 -> 56.1 TFLOP/s.
+// slots, and what bounds it is this tile's operand reads and the moves that
+// duplicate op(B)'s element: a register-only loop of it reaches 59.5 TFLOP/s (49
+// scalar), of a 16 x 8 tile 62.8, and cuBLAS 63.9 at 8192^3.  4096^3: 2654 -> 2543
+// us (54.0 TFLOP/s), 8192^3 NT 53.7 -> 56.1 TFLOP/s.
 // Operands are staged with cp.async; a K-fast global operand (op = T for A,
 // op = N for B) is transposed on the fly by per-element copies.
 #include <algorithm>

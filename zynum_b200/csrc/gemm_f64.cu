@@ -208,8 +208,8 @@ dgemm_dmma_kernel(int M, int N, int K, int k_chunk, double alpha, const double* 
 // which leaves its partial tile in shared memory and sums 64 / splits columns of all of
 // them through distributed shared memory, in rank order (deterministic).  Bound: launch
 // and memory latency.  Against 64 x 64 tiles with partials in a workspace and a reduction
-// kernel this saves the second launch (256^3 called back to back: 12.4 -> 9.9 us, bound by
-// the host's launches; on the device 6.5 / 6.6) and the partials' round trip through L2
+// kernel this saves the second launch (256^3 called back to back: 11.4 -> 9.3 us, bound by
+// the host's launches; on the device 6.6 / 6.8) and the partials' round trip through L2
 // (512^3: 16.0 -> 15.3 us, 128^3: 6.6 -> 5.1, 255^3 with odd leading dimensions 9.8 -> 7.1).
 // Eight warps of 32 x 16, fragments double-buffered in registers.
 constexpr int kCM = 64, kCN = 64, kCThreads = 256, kCStages = 4;
